@@ -186,66 +186,97 @@ __global__ void __launch_bounds__(256) k_build(BuildArgs a) {
     }
 }
 
-// FP64 edge coefficients of A for the FP64 rows (usv_internal.cuh: a_row):
-// e_nd = F_d 2/(rho_n + rho_d), F_d the face product of the direction tables,
-// by the same expressions a row used to evaluate on the fly (equal to the
-// last bits: the on-the-fly form may fuse the face product into the row's
-// FMAs); zero where the neighbour is missing.
-__global__ void __launch_bounds__(256) k_edges(OpView<double> op, double2* e64) {
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < op.n;
-         n += (long long)gridDim.x * blockDim.x) {
-        const Node p = decode(n, op.nx, op.ny);
-        const double rho = op.rec[n].x;
-        const double2 tx = op.T[0][p.i], ty = op.T[1][p.j], tz = op.T[2][p.k];
-        const double2 fyz = cmul(ty, tz), fxz = cmul(tx, tz), fxy = cmul(tx, ty);
-        const long long sy = op.nx, sz = (long long)op.nx * op.ny;
-        double2 e[6];
-        for (int d = 0; d < 6; ++d) e[d] = make_double2(0.0, 0.0);
-        auto edge = [&](int dir, long long m, double2 F) { e[dir] = cscale(F, 2.0 / (rho + op.rec[m].x)); };
-        if (p.i > 0) edge(0, n - 1, cmul(fyz, op.Q[0][p.i - 1]));
-        if (p.i < op.nx - 1) edge(1, n + 1, cmul(fyz, op.Q[0][p.i]));
-        if (p.j > 0) edge(2, n - sy, cmul(fxz, op.Q[1][p.j - 1]));
-        if (p.j < op.ny - 1) edge(3, n + sy, cmul(fxz, op.Q[1][p.j]));
-        if (p.k > 0) edge(4, n - sz, cmul(fxy, op.Q[2][p.k - 1]));
-        if (p.k < op.nz - 1) edge(5, n + sz, cmul(fxy, op.Q[2][p.k]));
-        for (int d = 0; d < 6; ++d) e64[6 * n + d] = e[d];
-    }
+// Row coefficients from the node records, one pass for all of them:
+//   e64   e_nd = F_d 2/(rho_n + rho_d) of A, F_d the face product of the
+//         direction tables (usv_internal.cuh: a_row; equal to the on-the-fly
+//         form to the last bits: that one may fuse the face product into the
+//         row's FMAs); zero where the neighbour is missing;
+//   cf/cb c_nd = R_n e_nd s_d of K and K' (conj(e_nd) and the adjoint
+//         scalings), formed in FP64 and rounded once to fp32 (and from there to
+//         packed bfloat16 {re, im} for the bfloat16 Arnoldi rows); zero for a
+//         fixed forward row and for a fixed neighbour of an adjoint row.
+// One FP64 division per edge: separate kernels that evaluated a whole row with
+// a unit vector per direction divided 36 times per node and direction set (at
+// 96^3: 39 us for e64, 111 + 132 us for K and K'). Stores go through shared
+// memory (a node's 96 / 48 / 24 bytes are written as whole lines).
+struct RowArrays {
+    double2* e64;
+    float4 *cff, *cfa;
+    uint2 *cbf, *cba;
+};
+constexpr int kRowThreads = 128;
+
+// Writes the block's W 16-byte words per node from shared memory, in order.
+template <int W>
+__device__ __forceinline__ void store_rows(const uint4* sm, uint4* dst, int count) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < W * count; q += kRowThreads) dst[q] = sm[q];
+    __syncthreads();
 }
 
-// Complex64 row coefficients c_nd = R_n e_nd s_d (conj(e_nd) and the adjoint
-// scalings for K'), evaluated in FP64 by the same row code as the FP64
-// operator with a unit value in direction d only, then rounded once to fp32
-// (and, for the bfloat16 Arnoldi rows, to packed bfloat16 {re, im}). The
-// complex64 rows (usv_internal.cuh: k_row_cf) then cost six complex
-// multiply-adds per node.
-template <bool ADJ>
-__global__ void __launch_bounds__(256) k_coef(OpView<double> op, float4* cf, uint2* cb) {
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < op.n;
-         n += (long long)gridDim.x * blockDim.x) {
-        const Node p = decode(n, op.nx, op.ny);
-        const long long sy = op.nx, sz = (long long)op.nx * op.ny;
-        const long long off[6] = {-1, 1, -sy, sy, -sz, sz};
-        const double4 me = op.rec[n];
+__global__ void __launch_bounds__(kRowThreads) k_rows(OpView<double> f, const double4* reca,
+                                                      RowArrays out) {
+    __shared__ __align__(16) uint4 sm[6 * kRowThreads];
+    const long long n0 = (long long)blockIdx.x * kRowThreads, n = n0 + threadIdx.x;
+    const int count = int(min((long long)kRowThreads, f.n - n0));
+    const bool in = n < f.n;
+    const long long sy = f.nx, sz = (long long)f.nx * f.ny;
+    const long long off[6] = {-1, 1, -sy, sy, -sz, sz};
+    double2 e[6];
+    bool has[6] = {false, false, false, false, false, false}, nbf[6];
+    bool fixed = false;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) e[d] = make_double2(0.0, 0.0), nbf[d] = false;
+    if (in) {
+        const Node p = decode(n, f.nx, f.ny);
+        const double rho = f.rec[n].x;
+        const double2 tx = f.T[0][p.i], ty = f.T[1][p.j], tz = f.T[2][p.k];
+        const double2 fyz = cmul(ty, tz), fxz = cmul(tx, tz), fxy = cmul(tx, ty);
+        fixed = node_fixed(f.soft, p.i, p.j, p.k, f.nx, f.ny, f.nz);
+        auto edge = [&](int dir, int i, int j, int k, double2 F) {
+            has[dir] = true;
+            nbf[dir] = node_fixed(f.soft, i, j, k, f.nx, f.ny, f.nz);
+            e[dir] = cscale(F, 2.0 / (rho + f.rec[n + off[dir]].x));
+        };
+        if (p.i > 0) edge(0, p.i - 1, p.j, p.k, cmul(fyz, f.Q[0][p.i - 1]));
+        if (p.i < f.nx - 1) edge(1, p.i + 1, p.j, p.k, cmul(fyz, f.Q[0][p.i]));
+        if (p.j > 0) edge(2, p.i, p.j - 1, p.k, cmul(fxz, f.Q[1][p.j - 1]));
+        if (p.j < f.ny - 1) edge(3, p.i, p.j + 1, p.k, cmul(fxz, f.Q[1][p.j]));
+        if (p.k > 0) edge(4, p.i, p.j, p.k - 1, cmul(fxy, f.Q[2][p.k - 1]));
+        if (p.k < f.nz - 1) edge(5, p.i, p.j, p.k + 1, cmul(fxy, f.Q[2][p.k]));
+    }
+    double2* se = reinterpret_cast<double2*>(sm);
+#pragma unroll
+    for (int d = 0; d < 6; ++d) se[6 * threadIdx.x + d] = e[d];
+    store_rows<6>(sm, reinterpret_cast<uint4*>(out.e64 + 6 * n0), count);
+#pragma unroll
+    for (int adj = 0; adj < 2; ++adj) {
+        const double4* rec = adj ? reca : f.rec;
         float2 c[6];
-        for (int d = 0; d < 6; ++d) {
-            const double2 v = k_row_from<double, ADJ>(
-                op, p, me, make_double2(0.0, 0.0), [&](int dir, double4& r, double2& uv) {
-                    r = op.rec[n + off[dir]];
-                    uv = make_double2(dir == d ? 1.0 : 0.0, 0.0);
-                });
-            c[d] = make_float2(float(v.x), float(v.y));
-        }
         unsigned pk[6];
+#pragma unroll
         for (int d = 0; d < 6; ++d) {
+            double2 v = make_double2(0.0, 0.0);
+            if (has[d] && (adj ? !nbf[d] : !fixed)) {
+                const double4 r = rec[n + off[d]];
+                v = cscale(cmul(adj ? cconj(e[d]) : e[d], make_double2(r.z, r.w)), rec[n].y);
+            }
+            c[d] = make_float2(float(v.x), float(v.y));
             const __nv_bfloat162 h = __floats2bfloat162_rn(c[d].x, c[d].y);
             pk[d] = *reinterpret_cast<const unsigned*>(&h);
         }
-        cb[3 * n] = make_uint2(pk[0], pk[1]);
-        cb[3 * n + 1] = make_uint2(pk[2], pk[3]);
-        cb[3 * n + 2] = make_uint2(pk[4], pk[5]);
-        cf[3 * n] = make_float4(c[0].x, c[0].y, c[1].x, c[1].y);
-        cf[3 * n + 1] = make_float4(c[2].x, c[2].y, c[3].x, c[3].y);
-        cf[3 * n + 2] = make_float4(c[4].x, c[4].y, c[5].x, c[5].y);
+        float2* sc = reinterpret_cast<float2*>(sm);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) sc[6 * threadIdx.x + d] = c[d];
+        store_rows<3>(sm, reinterpret_cast<uint4*>((adj ? out.cfa : out.cff) + 3 * n0), count);
+        // 24 bytes per node: one and a half 16-byte words, as 8-byte stores
+        unsigned* sp = reinterpret_cast<unsigned*>(sm);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) sp[6 * threadIdx.x + d] = pk[d];
+        __syncthreads();
+        uint2* cb = (adj ? out.cba : out.cbf) + 3 * n0;
+        for (int q = threadIdx.x; q < 3 * count; q += kRowThreads) cb[q] = reinterpret_cast<const uint2*>(sm)[q];
+        __syncthreads();
     }
 }
 
@@ -585,14 +616,10 @@ int usv_operator_build(const usv_scene* scene, const double* rho, const double* 
     a.flag = reinterpret_cast<int*>(buf + L.flag);
     k_build<<<grid_for(a.op.n), 256, 0, strm>>>(a);
     USV_CUDA_TRY(cudaGetLastError());
-    k_edges<<<grid_for(a.op.n), 256, 0, strm>>>(a.op, reinterpret_cast<double2*>(buf + L.e64));
-    USV_CUDA_TRY(cudaGetLastError());
-    k_coef<false><<<grid_for(a.op.n), 256, 0, strm>>>(
-        make_view<double>(s, op_buf, false), reinterpret_cast<float4*>(buf + L.cf32f),
-        reinterpret_cast<uint2*>(buf + L.cb16f));
-    k_coef<true><<<grid_for(a.op.n), 256, 0, strm>>>(
-        make_view<double>(s, op_buf, true), reinterpret_cast<float4*>(buf + L.cf32a),
-        reinterpret_cast<uint2*>(buf + L.cb16a));
+    const RowArrays rows{reinterpret_cast<double2*>(buf + L.e64),
+                         reinterpret_cast<float4*>(buf + L.cf32f), reinterpret_cast<float4*>(buf + L.cf32a),
+                         reinterpret_cast<uint2*>(buf + L.cb16f), reinterpret_cast<uint2*>(buf + L.cb16a)};
+    k_rows<<<unsigned((a.op.n + kRowThreads - 1) / kRowThreads), kRowThreads, 0, strm>>>(a.op, a.rec64a, rows);
     USV_CUDA_TRY(cudaGetLastError());
     int flag = 0;
     USV_CUDA_TRY(cudaMemcpyAsync(&flag, a.flag, sizeof(int), cudaMemcpyDeviceToHost, strm));

@@ -49,13 +49,63 @@ k_blend(int nx, int ny, int nz, double dx, const double* sdf, double cx, double 
     }
 }
 
-// One CTA per emitter; each thread owns one node of the emitter's bounding
-// box and gathers, in the reference's summation order (corner-major, then
-// quadrature order), the bilinear masses that land on it. Deterministic, no
-// atomics.
-__global__ void __launch_bounds__(256)
+// Aperture deposition: one CTA per emitter gathers, in the reference's
+// summation order (corner-major, then quadrature order), the bilinear masses
+// that land on each node of the emitter's bounding box. Deterministic, no
+// atomics on the masses.
+//
+// The order makes each node one chain of additions, so the parallelism is one
+// warp per node. The grid cell of every quadrature point is found once per
+// CTA (two FP64 divides per point) and the points are listed by cell in
+// shared memory, in quadrature order (one warp per cell compacts the matching
+// keys); a node's warp walks the lists of its four cells, forms 32 weights at
+// a time, one per lane, and adds them in order. A box of more than kDepCells
+// cells (an aperture wider than about 40 nodes) has no room for the lists: its
+// warps scan the keys for each cell instead. Bounded by instruction issue;
+// 256 emitters of 16384 points (96^3 scene): 16.4 ms with one thread per node
+// testing every point against its node, 0.58 ms with the scan, 0.36 ms with
+// the lists.
+constexpr int kDepThreads = 512;
+constexpr int kDepWarps = kDepThreads / 32;
+constexpr int kDepBlock = 16384;        // quadrature points per pass
+constexpr int kDepCells = 2048;
+constexpr int kDepQueue = 128 + 32;     // one scan step appends at most 128 points
+struct DepShared {
+    double2 term[kDepWarps][32];
+    int key[kDepBlock];                 // (cell x - x0 + 1) + (cell y - y0 + 1) (bw + 1), -1: outside
+    int first[kDepCells + 1];           // list of cell c: points[first[c]] .. points[first[c + 1] - 1]
+    union {
+        unsigned short points[kDepBlock];
+        unsigned short queue[kDepWarps][kDepQueue];
+    };
+};
+
+// Positions (quadrature order) of the keys equal to `want` among the 128 from
+// `k` on, four per lane: put(index, rank) for each; returns their number.
+template <typename Put>
+__device__ __forceinline__ int match_keys(const int* key, int k, int nk4, int want, Put&& put) {
+    const int lane = threadIdx.x & 31;
+    int4 kv = make_int4(-1, -1, -1, -1);
+    if (k + 4 * lane < nk4) kv = *reinterpret_cast<const int4*>(key + k + 4 * lane);
+    const bool h0 = kv.x == want, h1 = kv.y == want, h2 = kv.z == want, h3 = kv.w == want;
+    if (!__any_sync(0xffffffffu, h0 || h1 || h2 || h3)) return 0;
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned m0 = __ballot_sync(0xffffffffu, h0), m1 = __ballot_sync(0xffffffffu, h1);
+    const unsigned m2 = __ballot_sync(0xffffffffu, h2), m3 = __ballot_sync(0xffffffffu, h3);
+    int pos = __popc(m0 & below) + __popc(m1 & below) + __popc(m2 & below) + __popc(m3 & below);
+    if (h0) put(k + 4 * lane, pos++);
+    if (h1) put(k + 4 * lane + 1, pos++);
+    if (h2) put(k + 4 * lane + 2, pos++);
+    if (h3) put(k + 4 * lane + 3, pos++);
+    return __popc(m0) + __popc(m1) + __popc(m2) + __popc(m3);
+}
+
+__global__ void __launch_bounds__(kDepThreads)
 k_deposit(int nx, int ny, double dx, const double* centers, const double* qx,
           const double* qy, const double* qw, int q, double diameter, double* masses) {
+    extern __shared__ __align__(16) unsigned char dep_smem[];
+    DepShared& sm = *reinterpret_cast<DepShared*>(dep_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m = blockIdx.x;
     const double cx = centers[3 * m], cy = centers[3 * m + 1];
     const int x0 = int(floor((cx - 0.5 * diameter) / dx)) - 1;
@@ -63,22 +113,109 @@ k_deposit(int nx, int ny, double dx, const double* centers, const double* qx,
     const int x1 = int(floor((cx + 0.5 * diameter) / dx)) + 2;
     const int y1 = int(floor((cy + 0.5 * diameter) / dx)) + 2;
     const int bw = x1 - x0 + 1, bh = y1 - y0 + 1;
+    const int cells = (bw + 1) * (bh + 1);
+    const bool lists = cells <= kDepCells;
     double* col = masses + (long long)m * nx * ny;
-    for (int t = threadIdx.x; t < bw * bh; t += blockDim.x) {
-        const int ix = x0 + t % bw, iy = y0 + t / bw;
-        if (ix < 0 || iy < 0 || ix >= nx || iy >= ny) continue;
-        double acc = 0.0;
-        for (int corner = 0; corner < 4; ++corner) {
-            const int a = corner >> 1, b = corner & 1;
-            for (int k = 0; k < q; ++k) {
-                const double px = (cx + qx[k]) / dx, py = (cy + qy[k]) / dx;
-                const double fx0 = floor(px), fy0 = floor(py);
-                if (int(fx0) + a != ix || int(fy0) + b != iy) continue;
-                const double fx = px - fx0, fy = py - fy0;
-                acc += qw[k] * (a ? fx : 1.0 - fx) * (b ? fy : 1.0 - fy);
+    double2* term = sm.term[warp];
+    for (int corner = 0; corner < 4; ++corner) {
+        const int a = corner >> 1, b = corner & 1;
+        for (int k0 = 0; k0 < q; k0 += kDepBlock) {
+            const int nk = min(kDepBlock, q - k0), nk4 = (nk + 3) & ~3;
+            if (corner == 0 || q > kDepBlock) {
+                __syncthreads();  // every warp is done with the previous block
+                if (lists)
+                    for (int c = threadIdx.x; c <= cells; c += kDepThreads) sm.first[c] = 0;
+                __syncthreads();
+                for (int k = threadIdx.x; k < nk4; k += kDepThreads) {
+                    int v = -1;
+                    if (k < nk) {
+                        // a node takes the point from the cells at its own and
+                        // the previous index, so the box is widened by one cell
+                        const long long rx = (long long)int(floor((cx + qx[k0 + k]) / dx)) - x0 + 1;
+                        const long long ry = (long long)int(floor((cy + qy[k0 + k]) / dx)) - y0 + 1;
+                        if (rx >= 0 && rx <= bw && ry >= 0 && ry <= bh) v = int(rx + ry * (bw + 1));
+                    }
+                    sm.key[k] = v;
+                    if (lists && v >= 0) atomicAdd(&sm.first[v + 1], 1);
+                }
+                __syncthreads();
+                if (lists) {
+                    if (warp == 0) {  // counts to list starts
+                        int run = 0;
+                        for (int c0 = 1; c0 <= cells; c0 += 32) {
+                            const int c = c0 + lane;
+                            int v = c <= cells ? sm.first[c] : 0;
+#pragma unroll
+                            for (int o = 1; o < 32; o <<= 1) {
+                                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                                if (lane >= o) v += u;
+                            }
+                            if (c <= cells) sm.first[c] = run + v;
+                            run += __shfl_sync(0xffffffffu, v, 31);
+                        }
+                    }
+                    __syncthreads();
+                    for (int c = warp; c < cells; c += kDepWarps) {
+                        int pos = sm.first[c];
+                        const int end = sm.first[c + 1];
+                        for (int k = 0; k < nk4 && pos < end; k += 128)
+                            pos += match_keys(sm.key, k, nk4, c, [&](int i, int rank) {
+                                sm.points[pos + rank] = (unsigned short)i;
+                            });
+                    }
+                    __syncthreads();
+                }
+            }
+            for (int t = warp; t < bw * bh; t += kDepWarps) {
+                const int ix = x0 + t % bw, iy = y0 + t / bw;
+                if (ix < 0 || iy < 0 || ix >= nx || iy >= ny) continue;
+                const int want = (t % bw + 1 - a) + (t / bw + 1 - b) * (bw + 1);
+                double acc = col[(long long)iy * nx + ix];
+                auto add = [&](const unsigned short* list, int count) {  // count <= 32
+                    if (lane < count) {
+                        const int k = k0 + list[lane];
+                        const double px = (cx + qx[k]) / dx, py = (cy + qy[k]) / dx;
+                        const double fx = px - floor(px), fy = py - floor(py);
+                        term[lane] = make_double2(qw[k] * (a ? fx : 1.0 - fx), b ? fy : 1.0 - fy);
+                    }
+                    __syncwarp();
+                    if (count == 32) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) acc = fma(term[i].x, term[i].y, acc);
+                    } else {
+                        for (int i = 0; i < count; ++i) acc = fma(term[i].x, term[i].y, acc);
+                    }
+                    __syncwarp();
+                };
+                if (lists) {
+                    const int end = sm.first[want + 1];
+                    for (int i = sm.first[want]; i < end; i += 32) add(sm.points + i, min(32, end - i));
+                } else {
+                    unsigned short* queue = sm.queue[warp];
+                    int n = 0;  // queued points
+                    for (int k = 0; k < nk4; k += 128) {
+                        const int got = match_keys(sm.key, k, nk4, want, [&](int i, int rank) {
+                            queue[n + rank] = (unsigned short)i;
+                        });
+                        if (got == 0) continue;
+                        n += got;
+                        __syncwarp();
+                        int head = 0;
+                        for (; n - head >= 32; head += 32) add(queue + head, 32);
+                        if (head > 0) {  // fewer than 32 left: move them to the front
+                            n -= head;
+                            const unsigned short v = lane < n ? queue[head + lane] : (unsigned short)0;
+                            __syncwarp();
+                            if (lane < n) queue[lane] = v;
+                            __syncwarp();
+                        }
+                    }
+                    if (n > 0) add(queue, n);
+                }
+                if (lane == 0) col[(long long)iy * nx + ix] = acc;
+                __syncwarp();
             }
         }
-        col[(long long)iy * nx + ix] = acc;
     }
 }
 
@@ -86,35 +223,49 @@ k_deposit(int nx, int ny, double dx, const double* centers, const double* qx,
 __global__ void k_source_check(int nx, int ny, int m_emitters, const double* masses,
                                const double2* Tx, const double2* Ty, const double2* Tz,
                                unsigned soft, int nz, int* flag) {
-    const long long nxy = (long long)nx * ny;
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nxy;
-         n += (long long)gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int m = 0; m < m_emitters; ++m) s += fabs(masses[m * nxy + n]);
-        if (s <= 0) continue;
-        const int i = int(n % nx), j = int(n / nx);
+    // (a node counts as soon as one emitter deposits there, so every mass is
+    // tested by itself: one load per thread instead of a loop over emitters)
+    const long long nxy = (long long)nx * ny, total = nxy * m_emitters;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
+         q += (long long)gridDim.x * blockDim.x) {
+        if (fabs(masses[q]) <= 0) continue;
+        const int n = int(q % nxy);
+        const int i = n % nx, j = n / nx;
         if (Tx[i].y + Ty[j].y + Tz[0].y > 0) atomicOr(flag, 1);
         if (node_fixed(soft, i, j, 0, nx, ny, nz)) atomicOr(flag, 2);
     }
 }
 
+// Right-hand sides: the first `plane_ctas` CTAs of a column form its z = 0
+// plane (one thread per node), the others clear kRhsZero nodes each. Bounded
+// by the 16 B per node written.
+constexpr int kRhsZero = 4096;
 __global__ void __launch_bounds__(256)
 k_source_rhs(long long nxy, long long N, int m_emitters, const double* masses,
-             const double2* coeff, double scale, double2* rhs, long long ld) {
+             const double2* coeff, double scale, double2* rhs, long long ld, int plane_ctas) {
     const int b = blockIdx.y;
     const double2* cb = coeff + (long long)b * m_emitters;
     double2* out = rhs + b * ld;
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < N;
-         n += (long long)gridDim.x * blockDim.x) {
-        double2 acc = make_double2(0.0, 0.0);
-        if (n < nxy) {
-            for (int m = 0; m < m_emitters; ++m) {
-                const double w = masses[m * nxy + n];
-                if (w != 0.0) acc = cadd(acc, cscale(cb[m], scale * w));
-            }
-        }
-        out[n] = acc;
+    if (int(blockIdx.x) >= plane_ctas) {
+        const long long z0 = nxy + (long long)(blockIdx.x - plane_ctas) * kRhsZero + threadIdx.x;
+#pragma unroll
+        for (int u = 0; u < kRhsZero / 256; ++u)
+            if (z0 + 256 * u < N) out[z0 + 256 * u] = make_double2(0.0, 0.0);
+        return;
     }
+    const long long n = blockIdx.x * 256LL + threadIdx.x;
+    if (n >= nxy) return;
+    double2 acc = make_double2(0.0, 0.0);
+    // sixteen masses in flight per thread; added in emitter order
+    for (int m0 = 0; m0 < m_emitters; m0 += 16) {
+        double w[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) w[u] = m0 + u < m_emitters ? masses[(m0 + u) * nxy + n] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (w[u] != 0.0) acc = cadd(acc, cscale(cb[m0 + u], scale * w[u]));
+    }
+    out[n] = acc;
 }
 
 __global__ void __launch_bounds__(256)
@@ -251,12 +402,14 @@ int usv_source_masses(const usv_scene* scene, const void* op_buf,
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
     const long long nxy = (long long)s.nx * s.ny;
     USV_CUDA_TRY(cudaMemsetAsync(masses, 0, sizeof(double) * (nxy * m_emitters + 1), strm));
-    k_deposit<<<m_emitters, 256, 0, strm>>>(s.nx, s.ny, s.dx, centers_dev, quad_x, quad_y, quad_w,
-                                            q_points, diameter, masses);
+    USV_CUDA_TRY(cudaFuncSetAttribute(k_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(sizeof(DepShared))));
+    k_deposit<<<m_emitters, kDepThreads, sizeof(DepShared), strm>>>(s.nx, s.ny, s.dx, centers_dev, quad_x,
+                                                           quad_y, quad_w, q_points, diameter, masses);
     USV_CUDA_TRY(cudaGetLastError());
     const OpView<double> op = make_view<double>(s, op_buf, false);
     int* flag = reinterpret_cast<int*>(masses + nxy * m_emitters);
-    k_source_check<<<grid1(nxy), 256, 0, strm>>>(s.nx, s.ny, m_emitters, masses, op.T[0],
+    k_source_check<<<grid1(nxy * m_emitters), 256, 0, strm>>>(s.nx, s.ny, m_emitters, masses, op.T[0],
                                                  op.T[1], op.T[2], op.soft, s.nz, flag);
     USV_CUDA_TRY(cudaGetLastError());
     int h = 0;
@@ -277,10 +430,12 @@ int usv_source_rhs(const usv_scene* scene, const double* masses, int m_emitters,
     const long long N = (long long)s.nx * s.ny * s.nz, nxy = (long long)s.nx * s.ny;
     if (ld < N) return USV_ERR_ARG;
     const double scale = -2.0 * M_PI / (rho_ref * s.dx * s.dx * s.dx);
-    dim3 grid(grid1(N), nrhs);
+    const long long plane_ctas = (nxy + 255) / 256;
+    const long long zero_ctas = (N - nxy + kRhsZero - 1) / kRhsZero;
+    dim3 grid(unsigned(plane_ctas + zero_ctas), nrhs);
     k_source_rhs<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         nxy, N, m_emitters, masses, reinterpret_cast<const double2*>(coeff), scale,
-        static_cast<double2*>(rhs), ld);
+        static_cast<double2*>(rhs), ld, int(plane_ctas));
     USV_CUDA_TRY(cudaGetLastError());
     return USV_OK;
 }

@@ -387,7 +387,7 @@ __device__ __forceinline__ void k_coefs_from(const OpView<float>& op, Node p, fl
              ADJ && node_fixed(op.soft, p.i, p.j, p.k + 1, op.nx, op.ny, op.nz));
 }
 
-// Complex64 row from the precomputed coefficients (operator.cu: k_coef):
+// Complex64 row from the precomputed coefficients (operator.cu: k_rows):
 // y = u_n + sum_d c_nd u_d over the six neighbour directions. A missing
 // neighbour (grid edge) and every edge of a fixed forward row carry a zero
 // coefficient, so their loads are redirected to u_n, which exists and is finite.
@@ -608,7 +608,7 @@ __device__ __forceinline__ double2 a_row(const OpView<double>& op,
     if (!H && fixed) return ABS ? make_double2(cabs(xn), 0.0) : xn;
     const double2 d = op.d[n];
     double2 acc = ABS ? make_double2(cabs(d) * cabs(xn), 0.0) : (H ? cmulc(d, xn) : cmul(d, xn));
-    const double2* en = op.e64 + 6 * n;  // k_edges: F_d 2/(rho_n + rho_d)
+    const double2* en = op.e64 + 6 * n;  // k_rows: F_d 2/(rho_n + rho_d)
     auto edge = [&](int dir, long long m, bool nb_fixed) {
         if (H && nb_fixed) return;
         const double2 e = en[dir];
