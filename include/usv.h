@@ -108,7 +108,9 @@ typedef struct usv_scene {
  * 2 least squares, 3 solution update, 4 FP64 residual, 5 final gates,
  * 6 new recycled pair, 7 projection on the recycled space and the inner
  * products of the harmonic Ritz step. `launches` counts measured intervals
- * (a projection interval holds two kernels). */
+ * (a projection interval holds two kernels). Solves whose Arnoldi steps run in
+ * one launch per cycle report that launch, projection and orthogonalisation
+ * included, under family 0. */
 #define USV_KFAMILIES 8
 typedef struct usv_gmres_profile {
     int32_t launches[USV_KFAMILIES];

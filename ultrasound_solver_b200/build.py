@@ -21,9 +21,9 @@ CSRC = PKG / "csrc"
 INCLUDE = ROOT / "include"
 LIBDIR = PKG / "_lib"
 LIBNAME = "libusv_b200.so"
-SOURCES = ("operator.cu", "gmres.cu", "scene.cu", "basis.cu", "losses.cu", "surface.cu",
+SOURCES = ("operator.cu", "gmres.cu", "cycle.cu", "scene.cu", "basis.cu", "losses.cu", "surface.cu",
            "dense.cpp")
-HEADERS = ("usv_internal.cuh", "dense.h")
+HEADERS = ("usv_internal.cuh", "krylov.cuh", "dense.h")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -28,123 +28,16 @@
 #include <type_traits>
 #include <vector>
 
+#include "cycle.cuh"
 #include "dense.h"
-#include "usv_internal.cuh"
-
-#define USV_MAX_RESTART 112  // keeps the m x (m+1) least-squares tile in shared memory
 
 static_assert(sizeof(usv_gmres_params) == 80, "usv_gmres_params layout (include/usv.h)");
 
 namespace usv {
 
-enum { ST_ACTIVE = 0, ST_CONVERGED = 1, ST_MAXITER = 2, ST_NONFINITE = 3,
-       ST_DEVICE_TIMEOUT = 4 };  // a bounded device-side wait ran out
-
-// Per-RHS control words of a recycled (GCRO-DR) cycle, written by the host
-// before each cycle.
-enum {
-    CW_KC = 0,      // recycled vectors used by this cycle (0 or k)
-    CW_PAIR,        // pair buffer (U, C) used by this cycle
-    CW_VBUF,        // Krylov buffer of this cycle
-    CW_COMBINE,     // 1: build pair CW_DST at the start of this cycle
-    CW_SRC_PAIR,    // pair used by the cycle whose data builds the new pair
-    CW_SRC_VBUF,    // its Krylov buffer
-    CW_SRC_KC,      // its recycled count
-    CW_DST,         // pair buffer written by the combine
-    CW_HARVEST,     // 1: this cycle's data feeds a harmonic Ritz step
-    kCtl
-};
-constexpr int kPairBufs = 3;   // pairs in use: this cycle's, the source cycle's, the new one
-constexpr int kVBufs = 2;      // Krylov buffers: this cycle's and the previous cycle's
-
-struct GState {
-    int m, nblk, chunk, full_cycles, maxiter;
-    int nchunk;        // node chunks of `chunk` nodes; CTAs loop over them (grid <= nblk)
-    int ps;            // partial-sum slots per CTA
-    long long n;
-    long long nv;      // Krylov vector stride: n rounded up to 64 (512-B aligned pairs)
-    double rtol;
-    double2* partial;  // [B][nblk][ps], one row per CTA of the launch
-    double2* H;        // [B][m][m+1]  column j, rows 0..m
-    double* gc;        // [B][m]
-    double2* gs;       // [B][m]
-    double2* g;        // [B][m+1]
-    double2* y;        // [B][m]   (y_t * sigma_t)
-    double* sigma;     // [B][m+1]
-    double* bnorm;     // [B]
-    double* atol;      // [B]
-    double* wnorm;     // [B]
-    double* gates;     // [B][4]
-    double* hist;      // [B][hcap] ||r||/||Rb|| at each restart test
-    int hcap;
-    int* status;       // [B]
-    int* cycles;       // [B]
-    int* iters;        // [B]
-    int* len;          // [B]
-    int* ended;        // [B]
-    unsigned* counter; // [B]
-    // recycling (GCRO-DR), kr > 0 only
-    int kr;            // recycled vectors k
-    int hb_len;        // doubles per RHS in the host-read block
-    long long vstride; // elements between the Krylov buffers (B (m+1) nv)
-    long long pstride; // elements between pair buffers (B k nv)
-    void* Ubuf;        // [kPairBufs][B][k][nv] U, K U = C
-    void* Cbuf;        // [kPairBufs][B][k][nv] C, orthonormal
-    int* ctl;          // [B][kCtl]
-    double2* coef;     // [B][k + m + 1][2k] combine coefficients
-    double* hb;        // [B][hb_len] read by the host after each cycle:
-                       //   raw G columns [m][m+1] complex, bd [m+1][k] complex,
-                       //   sigma [m+1], d [k], then len, kc
-    double* dU;        // [kPairBufs][B][k] 1/||U_i||
-    double2* alpha;    // [B][k] projection C^H r of the cycle's first residual
-    int* klast;        // [B] recycled count of the last finished cycle
-    int* started;      // [B]
-    const struct SceneSlot* slots;  // [B] multi-scene solves: the scene of each RHS
-};
-
-// Scene of one right-hand side of a multi-scene solve (usv_gmres_solve_scenes):
-// the operator views, node count and chunk count of that scene and the node
-// steps of the 256- and kDotsThreads-thread kernels. Kernels instantiated
-// with MS = true read their scene from here (blockIdx.y = right-hand side);
-// single-scene kernels take it from their arguments.
-struct SceneSlot {
-    OpView<double> op64;
-    OpView<float> op32;
-    long long n;
-    int nchunk;
-    Step step, step_d;
-};
-template <typename R> __device__ __forceinline__ const OpView<R>& slot_view(const SceneSlot& s);
-template <> __device__ __forceinline__ const OpView<double>& slot_view<double>(const SceneSlot& s) {
-    return s.op64;
-}
-template <> __device__ __forceinline__ const OpView<float>& slot_view<float>(const SceneSlot& s) {
-    return s.op32;
-}
-// CTAs of the launch that work for right-hand side b: all of them for a
-// single scene; for a multi-scene batch a share proportional to the RHS's
-// scene size (the grid is sized for the largest scene), at least one.
-template <bool MS> __device__ __forceinline__ int rhs_ctas(const GState& g, int b) {
-    if constexpr (MS) {
-        const long long c = ((long long)gridDim.x * g.slots[b].n + g.n - 1) / g.n;
-        return int(c < 1 ? 1 : c);
-    } else {
-        return int(gridDim.x);
-    }
-}
-
-
-// host-read block offsets (in doubles)
-__host__ __device__ __forceinline__ int hb_graw(int) { return 0; }
-__host__ __device__ __forceinline__ int hb_bd(int m) { return 2 * m * (m + 1); }
-__host__ __device__ __forceinline__ int hb_sigma(int m, int k) { return hb_bd(m) + 2 * (m + 1) * k; }
-__host__ __device__ __forceinline__ int hb_d(int m, int k) { return hb_sigma(m, k) + m + 1; }
-__host__ __device__ __forceinline__ int hb_tail(int m, int k) { return hb_d(m, k) + k; }
-__host__ __device__ __forceinline__ int hb_size(int m, int k) { return hb_tail(m, k) + 2; }
-
 struct WsLayout {
     size_t V, partial, H, gc, gs, g, y, sigma, bnorm, atol, wnorm, gates, hist, status, cycles,
-        iters, len, ended, counter, state_begin, total;
+        iters, len, ended, counter, cyc_part, cyc_norm, cyc_tot, cyc_flag, cyc_epoch, state_begin, total;
     size_t U, C, bpart, coef, hb, dU, alpha, klast, started, ctl;  // recycling
     size_t slots;  // multi-scene solves: SceneSlot per right-hand side
 };
@@ -193,6 +86,11 @@ static WsLayout ws_layout(long long n, int m, int B, int nblk, size_t vec_bytes,
     L.len = take(sizeof(int) * B);
     L.ended = take(sizeof(int) * B);
     L.counter = take(sizeof(unsigned) * B);
+    L.cyc_part = take(sizeof(ulonglong2) * 2 * size_t(m + 2) * kCycMaxCtas);
+    L.cyc_norm = take(sizeof(ulonglong2) * kCycMaxCtas);
+    L.cyc_tot = take(sizeof(ulonglong2) * 2 * size_t(m + 2) * B);
+    L.cyc_flag = take(sizeof(unsigned long long) * kCycMaxCtas);
+    L.cyc_epoch = take(sizeof(unsigned long long));
     if (k > 0) {
         L.dU = take(sizeof(double) * size_t(kPairBufs) * B * k);
         L.alpha = take(sizeof(double2) * size_t(B) * k);
@@ -223,34 +121,6 @@ __device__ __forceinline__ double reduce_slot0(const GState& g, int b, double* s
     for (int q = threadIdx.x; q < nparts; q += blockDim.x)
         t += ld_cg(p + (long long)q * g.ps).x;
     return block_sum(t, sh);
-}
-
-// Vectors of RHS b's current cycle: t < kc are the recycled C_t (and U_t for
-// the solution update), the others Krylov slots of the cycle's buffer.
-template <typename S> struct CycleBasis {
-    S* V;        // Krylov slot 0
-    const S* C;  // C_0 of the cycle's pair (kc > 0)
-    const S* U;  // U_0 of the cycle's pair (kc > 0)
-    int kc;
-    int pair;
-};
-template <typename S>
-__device__ __forceinline__ CycleBasis<S> cycle_basis(S* V, const GState& g, int b) {
-    CycleBasis<S> cb;
-    cb.V = V + (long long)b * (g.m + 1) * g.nv;
-    cb.C = cb.U = cb.V;
-    cb.kc = 0;
-    cb.pair = 0;
-    if (g.kr > 0) {
-        const int* cw = g.ctl + b * kCtl;
-        cb.V += cw[CW_VBUF] * g.vstride;
-        cb.kc = cw[CW_KC];
-        cb.pair = cw[CW_PAIR] > 0 ? cw[CW_PAIR] : 0;
-        const long long po = cb.pair * g.pstride + (long long)b * g.kr * g.nv;
-        cb.C = static_cast<const S*>(g.Cbuf) + po;
-        cb.U = static_cast<const S*>(g.Ubuf) + po;
-    }
-    return cb;
 }
 
 // ------------------------------------------------------------ residual
@@ -428,24 +298,6 @@ __device__ __forceinline__ void stage_vector(uint4* stg, const C2* base, int t, 
     }
     cp_async_commit();
 }
-
-// Arithmetic of the basis passes per storage type. bfloat16 values (8-bit
-// mantissa) are combined in fp32: their products, the orthogonalisation
-// update and per-lane partial sums of at most a few dozen terms are far more
-// precise than the stored values; every reduction across lanes, CTAs and
-// chunks stays FP64. complex64 and complex128 bases use FP64 throughout.
-// (Widening to FP64 costs conversion-unit throughput: with bfloat16 the FP64
-// dots saturated that unit in the Arnoldi kernel.)
-template <typename C2> struct MathT {
-    using T = double;
-    using T2 = double2;
-};
-template <> struct MathT<bf2> {
-    using T = float;
-    using T2 = float2;
-};
-__device__ __forceinline__ double2 to_d(double2 a);
-__device__ __forceinline__ float2 to_f(bf2 a) { return bf2_to_f2(a); }
 
 // Complex value c (0/1) of pair k of stage t % S (in the pass arithmetic).
 template <typename C2>
@@ -847,17 +699,6 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
     }
     if (!last_block_done(&g.counter[b], ncta)) return;
     dots_finish(g, b, j, proj, ncta);
-}
-
-// d = a * b + c on two fp32 lanes at once (PTX fma.rn.f32x2, sm_100)
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(d)
-        : "l"(*reinterpret_cast<const unsigned long long*>(&a)),
-          "l"(*reinterpret_cast<const unsigned long long*>(&b)),
-          "l"(*reinterpret_cast<const unsigned long long*>(&c)));
-    return *reinterpret_cast<const float2*>(&d);
 }
 
 // Last CTA of an orthogonalisation launch: beta = ||u_{j+1}|| from the
@@ -1278,28 +1119,81 @@ __global__ void __launch_bounds__(OrthBulk<S>::THREADS) k_orth_bulk(S* V, long l
 // ------------------------------------------------------------ least squares (once per cycle)
 // Back-substitution R y = g on the Givens-reduced Hessenberg, staged in
 // shared memory; y is stored pre-multiplied by sigma (the basis scales).
+// RAW (after the cycle kernel): the columns are the plain Hessenberg ones; the
+// Givens rotations of all columns are applied here first, one rotation at a
+// time to all later columns in parallel.
+template <bool RAW>
 __global__ void __launch_bounds__(128) k_lsq(GState g) {
     const int b = blockIdx.x;
+    if (RAW && b == 0 && threadIdx.x == 0) *g.cyc_epoch += g.m + 3;  // past every step of the cycle
     if (g.status[b] != ST_ACTIVE || !g.ended[b]) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int m = g.m, L = g.len[b];
-    double2* Rs = reinterpret_cast<double2*>(smem_raw);  // L x L, column-major
-    double2* gv = Rs + (size_t)L * L;
-    for (int idx = threadIdx.x; idx < L * L; idx += blockDim.x) {
-        const int k = idx / L, i = idx % L;
-        Rs[idx] = i <= k ? g.H[((long long)b * m + k) * (m + 1) + i] : make_double2(0.0, 0.0);
+    const int ldr = RAW ? L + 1 : L;
+    double2* Rs = reinterpret_cast<double2*>(smem_raw);  // ldr x L, column-major
+    double2* gv = Rs + (size_t)ldr * L;
+    for (int idx = threadIdx.x; idx < ldr * L; idx += blockDim.x) {
+        const int k = idx / ldr, i = idx % ldr;
+        Rs[idx] = i <= (RAW ? k + 1 : k) ? g.H[((long long)b * m + k) * (m + 1) + i] : make_double2(0.0, 0.0);
     }
-    for (int i = threadIdx.x; i < L; i += blockDim.x) gv[i] = g.g[(long long)b * (m + 1) + i];
+    for (int i = threadIdx.x; i < L + (RAW ? 1 : 0); i += blockDim.x) gv[i] = g.g[(long long)b * (m + 1) + i];
+    __syncthreads();
+    if constexpr (RAW) {
+        // (the columns t < kc of a recycled cycle are diagonal: no rotation)
+        for (int i = g.kr > 0 ? g.ctl[b * kCtl + CW_KC] : 0; i < L; ++i) {
+            // rotation zeroing beta: c = |a|/r, s = (a/|a|) beta/r, rho = (a/|a|) r
+            const double2 a = Rs[(size_t)i * ldr + i];
+            const double beta = Rs[(size_t)i * ldr + i + 1].x;
+            const double a2 = fma(a.x, a.x, a.y * a.y), r2 = fma(beta, beta, a2);
+            double c, r, rinv, ainv;
+            double2 sn = make_double2(1.0, 0.0), rho = make_double2(beta, 0.0);
+            if (a2 > 1e-280 && r2 < 1e280) {
+                // two independent reciprocal roots instead of a chain of two
+                // hypot and three divisions (a column's rotation is the serial
+                // part of this kernel)
+                ainv = rsqrt(a2), rinv = rsqrt(r2);
+                c = a2 * ainv * rinv, r = r2 * rinv;
+            } else {
+                const double aa = hypot(a.x, a.y);
+                r = hypot(aa, beta);
+                ainv = 1.0 / aa, rinv = 1.0 / r;
+                c = aa / r;
+            }
+            if (a.x != 0.0 || a.y != 0.0) {
+                const double2 ph = cscale(a, ainv);
+                sn = cscale(ph, beta * rinv);
+                rho = cscale(ph, r);
+            } else {
+                c = 0.0;
+            }
+            __syncthreads();
+            for (int j = i + int(threadIdx.x); j <= L; j += blockDim.x) {
+                if (j == i) {
+                    Rs[(size_t)i * ldr + i] = rho;
+                    Rs[(size_t)i * ldr + i + 1] = make_double2(0.0, 0.0);
+                } else {  // column j, or (j = L) the right-hand side
+                    double2* v = j < L ? Rs + (size_t)j * ldr + i : gv + i;
+                    const double2 x = v[0], y = v[1];
+                    v[0] = cadd(cscale(x, c), cmul(sn, y));
+                    v[1] = csub(cscale(y, c), cmulc(sn, x));
+                }
+            }
+            __syncthreads();
+        }
+    }
+    // back-substitution: 1/R_kk of all columns first (off the serial chain)
+    for (int k = threadIdx.x; k < L; k += blockDim.x)
+        Rs[(size_t)k * ldr + k] = cinv(Rs[(size_t)k * ldr + k]);
     __syncthreads();
     for (int k = L - 1; k >= 0; --k) {
         // y_k = g_k / R_kk (every thread computes it from shared memory)
-        const double2 yk = cmul(gv[k], cinv(Rs[(size_t)k * L + k]));
-        __syncthreads();
+        const double2 yk = cmul(gv[k], Rs[(size_t)k * ldr + k]);
         for (int i = threadIdx.x; i < k; i += blockDim.x)
-            gv[i] = csub(gv[i], cmul(Rs[(size_t)k * L + i], yk));
-        if (threadIdx.x == 0) gv[k] = yk;
+            gv[i] = csub(gv[i], cmul(Rs[(size_t)k * ldr + i], yk));
         __syncthreads();
     }
+    for (int k = threadIdx.x; k < L; k += blockDim.x) gv[k] = cmul(gv[k], Rs[(size_t)k * ldr + k]);
+    __syncthreads();
     if (g.kr == 0) {
         for (int i = threadIdx.x; i < L; i += blockDim.x)
             g.y[(long long)b * m + i] = cscale(gv[i], g.sigma[b * (m + 1) + i]);
@@ -2338,7 +2232,7 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
                                      cudaMemcpyHostToDevice, strm));
         g.slots = dslots;
     }
-    const size_t lsq_smem = sizeof(double2) * size_t(g.m) * (g.m + 1);
+    const size_t lsq_smem = sizeof(double2) * size_t(g.m + 1) * (g.m + 1);
     const size_t pipe_smem = Pipe<C2>::STAGED ? Pipe<C2>::BYTES : 16;
     const Step step = make_step(kThreads, s.nx, s.ny);
     const Step step_d = make_step(kDotsThreads, s.nx, s.ny);
@@ -2417,8 +2311,29 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
     if (int e = grid_for((const void*)k_update<S, MS>, kThreads, pipe_smem, grid_upd)) return e;
     if (int e = grid_for((const void*)k_gates<ADJ, MS>, 256, 0, grid_gates)) return e;
     if (lsq_smem > 48 * 1024)
-        USV_CUDA_TRY(cudaFuncSetAttribute(k_lsq, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(lsq_smem)));
+        for (auto* fn : {k_lsq<false>, k_lsq<true>})
+            USV_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              int(lsq_smem)));
+    // Short passes: the Arnoldi steps of a cycle in one cooperative launch
+    // (cycle.cu). It runs whole cycles only, and the selectable kernel forms
+    // and the CTA cap are those of the per-step kernels.
+    CyclePlan cyc;
+    {
+        std::vector<long long> sizes(B, g.n);
+        if constexpr (MS)
+            for (int b = 0; b < B; ++b) sizes[b] = (*slots)[b].n;
+        if (g.full_cycles && p.max_ctas == 0 &&
+            !(p.kernel_variant & (USV_GMRES_ORTH_CPASYNC | USV_GMRES_DOTS_C64_ROWS)))
+            USV_CUDA_TRY((cycle_plan<R, S, MS>(g.m, sizes.data(), B, sms, cyc)));
+    }
+    auto launch_steps = [&](cudaStream_t st) -> cudaError_t {
+        OpView<R> ov = opk;
+        C2* vp = V;
+        GState gs = g;
+        int nrhs = B, adj = ADJ ? 1 : 0, smem = int(cyc.smem);
+        void* args[] = {&ov, &vp, &gs, &nrhs, &adj, &smem};
+        return cudaLaunchCooperativeKernel(cyc.fn, dim3(cyc.ctas), dim3(kCycThreads), args, cyc.smem, st);
+    };
     const int kr = g.kr;
     dim3 grid_bd, grid_comb;
     size_t bd_smem = 0, comb_smem = 0;
@@ -2566,16 +2481,29 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
             fam_shared.push_back(nn * (sizeof(double4) + 7 * sizeof(double2)));
             fam_step.push_back(-1);
             fam_need.push_back(0);
-            USV_CUDA_TRY(launch_dots(st, 0, 1));
-            USV_CUDA_TRY(launch_orth(st, 0, 1));
+            if (!cyc.ctas) {
+                USV_CUDA_TRY(launch_dots(st, 0, 1));
+                USV_CUDA_TRY(launch_orth(st, 0, 1));
+                USV_CUDA_TRY(mark(st, k++, capturing));
+                fam.push_back(7);
+                fam_bytes.push_back(nn * vb * (2.0 * kr + 3));
+                fam_shared.push_back(0.0);
+                fam_step.push_back(-1);
+                fam_need.push_back(1);
+            }
+        }
+        if (cyc.ctas) {
+            // projection and all Arnoldi steps; bytes of the steps kc..m-1 are
+            // added when the interval is read
+            USV_CUDA_TRY(launch_steps(st));
             USV_CUDA_TRY(mark(st, k++, capturing));
-            fam.push_back(7);
-            fam_bytes.push_back(nn * vb * (2.0 * kr + 3));
+            fam.push_back(0);
+            fam_bytes.push_back(0.0);
             fam_shared.push_back(0.0);
             fam_step.push_back(-1);
-            fam_need.push_back(1);
+            fam_need.push_back(4);
         }
-        for (int j = 0; j < g.m; ++j) {
+        for (int j = cyc.ctas ? g.m : 0; j < g.m; ++j) {
             USV_CUDA_TRY(launch_dots(st, j, 0));
             USV_CUDA_TRY(mark(st, k++, capturing));
             fam.push_back(0);
@@ -2594,7 +2522,8 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
             fam_step.push_back(j);
             fam_need.push_back(0);
         }
-        k_lsq<<<B, 128, lsq_smem, st>>>(g);
+        if (cyc.ctas) k_lsq<true><<<B, 128, lsq_smem, st>>>(g);
+        else k_lsq<false><<<B, 128, lsq_smem, st>>>(g);
         USV_CUDA_TRY(mark(st, k++, capturing));
         fam.push_back(2);
         fam_bytes.push_back(0.0);
@@ -2651,8 +2580,15 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
                               (fam_need[i] == 1 && meas_kc == 0) ||
                               (fam_need[i] == 2 && !meas_combine) ||
                               (fam_need[i] == 3 && (meas_kc == 0 || !meas_harvest));
-            if (!idle && active_counts[0] > 0)
-                prof->bytes[fam[i]] += fam_bytes[i] * active_counts[0] + fam_shared[i];
+            double by = fam_bytes[i], sh = fam_shared[i];
+            if (fam_need[i] == 4) {
+                if (meas_kc > 0) by += nn * vb * (2.0 * kr + 3);
+                for (int j = meas_kc; j < g.m; ++j) {
+                    by += nn * vb * (2.0 * j + 5);
+                    sh += nn * (sizeof(R) == 8 ? 96.0 : (rows16 ? 24.0 : 48.0));
+                }
+            }
+            if (!idle && active_counts[0] > 0) prof->bytes[fam[i]] += by * active_counts[0] + sh;
         }
         return USV_OK;
     };
@@ -2881,6 +2817,11 @@ static GState make_state(char* ws, const WsLayout& L, const usv_gmres_params* pa
     g.len = reinterpret_cast<int*>(ws + L.len);
     g.ended = reinterpret_cast<int*>(ws + L.ended);
     g.counter = reinterpret_cast<unsigned*>(ws + L.counter);
+    g.cyc_part = reinterpret_cast<ulonglong2*>(ws + L.cyc_part);
+    g.cyc_norm = reinterpret_cast<ulonglong2*>(ws + L.cyc_norm);
+    g.cyc_tot = reinterpret_cast<ulonglong2*>(ws + L.cyc_tot);
+    g.cyc_flag = reinterpret_cast<unsigned long long*>(ws + L.cyc_flag);
+    g.cyc_epoch = reinterpret_cast<unsigned long long*>(ws + L.cyc_epoch);
     g.ps = partial_slots(m, kr);
     g.kr = kr;
     if (kr > 0) {
