@@ -786,11 +786,12 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
 // The smallest instance whose CTAs hold the largest share of nodes a launch can
 // see: all right-hand sides active. Measured per Arnoldi step of GMRES(30),
 // this kernel / one launch per pass (us; nodes over all right-hand sides):
-//   bfloat16   14.0 / 29.4 at 14 k, 17.6 / 32.4 at 262 k, 24.4 / 38.4 at 593 k, 38.2 / 50.6 at 1.19 M
+//   bfloat16   14.0 / 29.4 at 14 k, 17.6 / 32.4 at 262 k, 24.4 / 38.4 at 593 k, 38.2 / 50.6 at 1.19 M,
+//              69.7 / 77.1 at 1.77 M, 85.4 / 88.3 at 2.10 M
 //   complex64  14.4 / 34.2         23.0 / 37.2            39.5 / 53.8          82.4 / 86.7
 //   complex128 14.8 / 40.7         31.8 / 48.8            102  / 85.9
-// so bfloat16 and complex64 take it up to 8192 nodes per CTA and complex128 up
-// to 2048 (303 k nodes on 148 SMs).
+// so bfloat16 takes it up to 16384 nodes per CTA, complex64 up to 8192 and
+// complex128 up to 2048 (2.4 M, 1.2 M and 303 k nodes on 148 SMs).
 template <typename R, typename S, bool MS>
 cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePlan& plan) {
     plan = CyclePlan{};
@@ -815,7 +816,7 @@ cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePl
     take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 2 * U0>), Geo<S, 2 * U0>::MAX);
     if constexpr (sizeof(S) != 16)
         take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 4 * U0>), Geo<S, 4 * U0>::MAX);
-    if constexpr (sizeof(S) == 8)
+    if constexpr (sizeof(S) != 16)
         take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 8 * U0>), Geo<S, 8 * U0>::MAX);
     if (!fn) return cudaSuccess;
     const CycFixed<S> fix(m, max_nodes);
