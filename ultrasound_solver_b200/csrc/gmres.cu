@@ -839,7 +839,9 @@ __global__ void __launch_bounds__(kThreads) k_orth(S* V, long long N, GState g, 
     }
     __syncthreads();  // hs, hm visible
     double acc = 0.0;
-    for (int ch = blockIdx.x; ch < nchunk; ch += ncta) {
+    // last chunk first: the dots pass ended there, and what it read last is
+    // still in L2 (the next dots pass starts where this one ends)
+    for (int ch = nchunk - 1 - int(blockIdx.x); ch >= 0; ch -= ncta) {
         const long long n0 = (long long)ch * kChunk;
         const int len = int(min((long long)kChunk, N - n0));
         C2* w = cb.V + (long long)(j + 1) * g.nv + n0;
@@ -995,6 +997,8 @@ __global__ void __launch_bounds__(OrthBulk<S>::THREADS) k_orth_bulk(S* V, long l
     }
     __syncthreads();  // hs, hm, barriers visible
     const int tpc = j + 2;  // tiles per chunk: w, u_0 .. u_j
+    // (last chunk first: the dots pass ended there, and what it read last is
+    // still in L2; the next dots pass starts where this one ends)
     const int nmy = nchunk > int(blockIdx.x) ? int((nchunk - blockIdx.x + ncta - 1) / ncta) : 0;
     double acc = 0.0;
     if (warp == kThreads / 32) {
@@ -1003,7 +1007,7 @@ __global__ void __launch_bounds__(OrthBulk<S>::THREADS) k_orth_bulk(S* V, long l
             int q = 0;
             bool ok = true;
             for (int i = 0; i < nmy && ok; ++i) {
-                const long long n0 = (long long)(blockIdx.x + (long long)i * ncta) * kChunk;
+                const long long n0 = (nchunk - 1 - blockIdx.x - (long long)i * ncta) * kChunk;
                 const int len = int(min((long long)kChunk, N - n0));
                 const unsigned bytes = unsigned((size_t(len) * sizeof(C2) + 15) / 16 * 16);
                 for (int tt = 0; tt < tpc; ++tt, ++q) {
@@ -1031,7 +1035,7 @@ __global__ void __launch_bounds__(OrthBulk<S>::THREADS) k_orth_bulk(S* V, long l
     } else {
         int q = 0;
         for (int i = 0; i < nmy; ++i) {
-            const long long n0 = (long long)(blockIdx.x + (long long)i * ncta) * kChunk;
+            const long long n0 = (nchunk - 1 - blockIdx.x - (long long)i * ncta) * kChunk;
             const int len = int(min((long long)kChunk, N - n0));
             M2 u[kPairs][2];
             bool ok = true;
