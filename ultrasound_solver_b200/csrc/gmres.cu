@@ -431,8 +431,9 @@ constexpr int kDotUnroll = 8;
 constexpr int kDotsThreads = 512;
 
 template <typename Y, typename C2> __device__ __forceinline__ Y as_ys(C2 v) { return v; }
+// (complex64: carries the 2^896 that widen_scaled leaves to the other factor)
 template <> __device__ __forceinline__ double2 as_ys<double2, float2>(float2 v) {
-    return make_double2(v.x, v.y);
+    return make_double2(double(v.x) * kScaleUp, double(v.y) * kScaleUp);
 }
 
 template <typename C2> struct LaneLoad;
@@ -451,16 +452,33 @@ template <> struct LaneLoad<float2> {
     float4 r;
     __device__ __forceinline__ void load(const float2* p) { r = *reinterpret_cast<const float4*>(p); }
     __device__ __forceinline__ void zero() { r = make_float4(0.f, 0.f, 0.f, 0.f); }
-    __device__ __forceinline__ double2 get(int i) const {
-        return i ? make_double2(r.z, r.w) : make_double2(r.x, r.y);
+    __device__ __forceinline__ double2 get(int i) const {  // scaled by 2^-896
+        return i ? make_double2(widen_scaled(__float_as_uint(r.z)), widen_scaled(__float_as_uint(r.w)))
+                 : make_double2(widen_scaled(__float_as_uint(r.x)), widen_scaled(__float_as_uint(r.y)));
     }
 };
 template <> struct LaneLoad<double2> {
-    static constexpr int NL = 2;
-    double2 a, b;
-    __device__ __forceinline__ void load(const double2* p) { a = p[0]; b = p[1]; }
-    __device__ __forceinline__ void zero() { a = b = make_double2(0.0, 0.0); }
-    __device__ __forceinline__ double2 get(int i) const { return i ? b : a; }
+    // one node per lane: with two, a load touches half of each line it reads,
+    // and the L1 path bounded the kernel (97 x 90 x 83, 2 right-hand sides:
+    // 123.0 -> 118.8 us per launch)
+    static constexpr int NL = 1;
+    double2 a;
+    __device__ __forceinline__ void load(const double2* p) { a = *p; }
+    __device__ __forceinline__ void zero() { a = make_double2(0.0, 0.0); }
+    __device__ __forceinline__ double2 get(int) const { return a; }
+};
+// Place of node e of the chunk in the shared copy of w. complex64: even and odd
+// nodes in two planes (64 bytes off each other in the banks), so that the lanes
+// of a load read 16-byte words next to each other (128^3: 86.4 -> 82.0 us per
+// launch; grouping four vectors per load of w instead: 85.1, and slower for the
+// other types).
+template <typename C2, int DC> struct YsPlace {
+    static constexpr int SIZE = DC;
+    static __device__ __forceinline__ int at(int e) { return e; }
+};
+template <int DC> struct YsPlace<float2, DC> {
+    static constexpr int SIZE = DC + 4;
+    static __device__ __forceinline__ int at(int e) { return (e >> 1) + (e & 1) * (DC / 2 + 4); }
 };
 
 // Last CTA of a dots launch: sum the per-CTA partials of t = 0..j (the dots)
@@ -546,7 +564,8 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
     // others still read chunk c (one barrier per chunk, between the stencil
     // and the dots)
     constexpr int NBUF = std::is_same<C2, bf2>::value ? 2 : 1;
-    __shared__ __align__(16) YS ys_buf[NBUF][DC];
+    using Place = YsPlace<C2, DC>;
+    __shared__ __align__(16) YS ys_buf[NBUF][Place::SIZE];
     __shared__ double2 segsum[USV_MAX_RESTART + 2 > NT / 16 ? USV_MAX_RESTART + 2 : NT / 16];
     const long long N = op.n;
     const C2* uj = cb.V + (long long)j * g.nv;
@@ -602,13 +621,13 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
                         y = narrow<C2>(cscale(k_row<R, ADJ, S>(op, uj, n, p), sj));
                         w[n] = y;
                     }
-                    ys[e] = as_ys<YS>(y);
+                    ys[Place::at(e)] = as_ys<YS>(y);
                     advance(p, step, op.nx, op.ny);
                 }
             }
         } else {
             for (int e = threadIdx.x; e < DC; e += NT)
-                ys[e] = as_ys<YS>(e < len ? w[n0 + e] : from_d<C2>(make_double2(0.0, 0.0)));
+                ys[Place::at(e)] = as_ys<YS>(e < len ? w[n0 + e] : from_d<C2>(make_double2(0.0, 0.0)));
         }
         __syncthreads();
         constexpr int NL = LaneLoad<C2>::NL;
@@ -672,7 +691,7 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
                         const int q = min(qb + 32 * u, ngroups - 1);
 #pragma unroll
                         for (int c = 0; c < NL; ++c) {
-                            const M2 y = widen<M2>(ys[NL * q + c]);
+                            const M2 y = widen<M2>(ys[Place::at(NL * q + c)]);
                             const M2 av = a[u].get(c);
                             lre = fma(av.x, y.x, fma(av.y, y.y, lre));
                             lim = fma(av.x, y.y, fma(-av.y, y.x, lim));
@@ -682,7 +701,11 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
             } else {
                 for (int q = q0 + lane; q < q1; q += 32)
 #pragma unroll
-                    for (int c = 0; c < NL; ++c) lre += cabs2(widen<M2>(ys[NL * q + c]));
+                    for (int c = 0; c < NL; ++c) {
+                        M2 y = widen<M2>(ys[Place::at(NL * q + c)]);
+                        if constexpr (std::is_same<C2, float2>::value) y = cscale(y, kScaleDown);
+                        lre += cabs2(y);
+                    }
             }
             const double v = warp_sum_pair(double(lre), double(lim));
             if ((lane & 15) == 0) reinterpret_cast<double*>(&segsum[task])[lane >> 4] += v;

@@ -176,4 +176,87 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
     return *reinterpret_cast<const float2*>(&d);
 }
 
+// A float widened to double, scaled by 2^-896: the exponent field is moved,
+// not rebiased, which is exact for every finite value (zeros and denormals
+// included). Integer instructions: F2F.F64.F32 runs at 16 lanes per clock and
+// SM and bounded the complex64 passes (2 per value and pass). The other factor
+// of a product carries 2^896, or the sum is scaled back. Infinities and NaN
+// would turn finite here: only basis vectors whose norm has been found finite
+// are read this way; w is converted by F2F, once per step.
+__device__ __forceinline__ double widen_scaled(unsigned f) {
+    const long long t = (long long)(int)f * (1LL << 29);
+    return __hiloint2double(int(t >> 32) & int(0x8fffffff), int(t));
+}
+constexpr double kScaleUp = 0x1p896, kScaleDown = 0x1p-896;
+
+// Dots of w with several basis vectors at once: the 16-byte loads of w (shared
+// memory) serve kDotVecs vectors.
+constexpr int kDotVecs = 4;  // vectors of one dots task (they share its loads of w)
+// w in shared memory as the dots read it: packed bfloat16, or FP64.
+template <typename S> struct DotW { using T = S; };
+template <> struct DotW<float2> { using T = double2; };
+
+// the stored row value as the dots read it
+__device__ __forceinline__ bf2 dot_value(bf2 y) { return y; }
+__device__ __forceinline__ double2 dot_value(double2 y) { return y; }
+__device__ __forceinline__ double2 dot_value(float2 y) {
+    return make_double2(double(y.x) * kScaleUp, double(y.y) * kScaleUp);
+}
+
+// w of one 16-byte load's nodes, from shared memory to registers
+template <typename S> struct UnitW;
+template <> struct UnitW<bf2> {
+    uint4 y;
+    __device__ __forceinline__ explicit UnitW(const bf2* p) : y(*reinterpret_cast<const uint4*>(p)) {}
+};
+template <> struct UnitW<float2> {
+    double2 y[2];
+    __device__ __forceinline__ explicit UnitW(const double2* p) : y{p[0], p[1]} {}
+};
+template <> struct UnitW<double2> {
+    double2 y;
+    __device__ __forceinline__ explicit UnitW(const double2* p) : y(p[0]) {}
+};
+// re, im += conj(v) w over the nodes of one 16-byte load
+__device__ __forceinline__ void unit_dot(uint4 v, const UnitW<bf2>& w, float& re, float& im) {
+    float rr = re, ii = 0.f, ri = im, ir = 0.f;
+    bf_mac(rr, ii, ri, ir, v.x, w.y.x);
+    bf_mac(rr, ii, ri, ir, v.y, w.y.y);
+    bf_mac(rr, ii, ri, ir, v.z, w.y.z);
+    bf_mac(rr, ii, ri, ir, v.w, w.y.w);
+    re = rr + ii;
+    im = ri - ir;
+}
+__device__ __forceinline__ void unit_dot(uint4 v, const UnitW<float2>& w, double& re, double& im) {
+    // (w carries the 2^896 of widen_scaled)
+    const double2 a = make_double2(widen_scaled(v.x), widen_scaled(v.y));
+    const double2 b = make_double2(widen_scaled(v.z), widen_scaled(v.w));
+    re = fma(a.x, w.y[0].x, fma(a.y, w.y[0].y, fma(b.x, w.y[1].x, fma(b.y, w.y[1].y, re))));
+    im = fma(a.x, w.y[0].y, fma(-a.y, w.y[0].x, fma(b.x, w.y[1].y, fma(-b.y, w.y[1].x, im))));
+}
+__device__ __forceinline__ void unit_dot(uint4 v, const UnitW<double2>& w, double& re, double& im) {
+    const double2 a = *reinterpret_cast<const double2*>(&v);
+    re = fma(a.x, w.y.x, fma(a.y, w.y.y, re));
+    im = fma(a.x, w.y.y, fma(-a.y, w.y.x, im));
+}
+
+// Warp sums of the kDotVecs complex dots v of all lanes; every fourth lane
+// holds the total of value `index`.
+__device__ __forceinline__ double warp_sum_dots(double (&v)[2 * kDotVecs], int& index) {
+    const int lane = threadIdx.x & 31;
+    index = ((lane & 16) ? 4 : 0) + ((lane & 8) ? 2 : 0) + ((lane & 4) ? 1 : 0);
+#pragma unroll
+    for (int h = kDotVecs, bit = 16; h > 0; h >>= 1, bit >>= 1) {
+        const bool hi = lane & bit;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double keep = hi ? v[i + h] : v[i];
+            const double send = hi ? v[i] : v[i + h];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+    }
+    double t = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 2);
+    return t + __shfl_xor_sync(0xffffffffu, t, 1);
+}
+
 }  // namespace usv
