@@ -342,43 +342,71 @@ __global__ void __launch_bounds__(256, 4) k_apply_kc(OpView<float> op, const flo
 // thread divides: a CTA of 32 x 8 threads covers 32 nodes along x of a few
 // rows j of plane k. The R right-hand sides (nrhs rounded up to a power of
 // two) are split into G = R / NB groups of NB; a thread applies its node's
-// coefficients (loaded once) to the NB vectors b = g, g + G, ..., and each
-// warp holds 32 consecutive nodes (coalesced loads and stores); the G warps
-// of a row share its coefficient loads through L1.
+// coefficients to the NB vectors b = g, g + G, ..., and each warp holds 32
+// consecutive nodes (coalesced loads and stores). The rows' coefficients (48
+// bytes per node, contiguous along x) reach shared memory by bulk copies while
+// the threads load their vector values: read by the lanes themselves, 48 bytes
+// apart, they took most of the L1 path that bounds this kernel, once per group.
+// 128^3, per launch: 33.2 -> 29.0 us (2 right-hand sides), 49.6 -> 45.3 (4,
+// 5.2 TB/s), 94.8 -> 82.0 (8). Marching through z with the column's values in
+// registers was slower at every run length (64 us and up for 4).
 template <int R, int NB>
 __global__ void __launch_bounds__(256) k_apply_kc_rhs(OpView<float> op, const float2* __restrict__ x,
                                                       float2* __restrict__ y, long long ld, int nrhs) {
     constexpr int G = R / NB, kRows = 8 / G;
+    __shared__ __align__(128) float4 rows[kRows][3 * 32];
+    __shared__ unsigned long long bar;
     const int i = blockIdx.x * 32 + threadIdx.x;
-    const int g = threadIdx.y % G;
-    const int j = blockIdx.y * kRows + threadIdx.y / G;
+    const int g = threadIdx.y % G, row = threadIdx.y / G;
+    const int j0 = blockIdx.y * kRows, j = j0 + row;
     const int k = blockIdx.z;
-    if (i >= op.nx || j >= op.ny || g >= nrhs) return;
     const long long sy = op.nx, sz = (long long)op.nx * op.ny;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        mbar_init(&bar, 1);
+        mbar_fence_init();
+        const int nrow = min(kRows, op.ny - j0);
+        const unsigned bytes = unsigned(min(32, op.nx - int(blockIdx.x) * 32)) * 48u;
+        mbar_expect_tx(&bar, bytes * nrow);
+        for (int q = 0; q < nrow; ++q)
+            bulk_g2s(rows[q], op.cf + 3 * (blockIdx.x * 32 + sy * (j0 + q) + sz * k), bytes, &bar);
+    }
+    const bool in = i < op.nx && j < op.ny && g < nrhs;
     const long long n = i + sy * j + sz * k;
-    const float4* cf = op.cf + 3 * n;
-    const float4 c01 = __ldg(cf), c23 = __ldg(cf + 1), c45 = __ldg(cf + 2);
     const long long o0 = i > 0 ? -1 : 0, o1 = i < op.nx - 1 ? 1 : 0;
     const long long o2 = j > 0 ? -sy : 0, o3 = j < op.ny - 1 ? sy : 0;
     const long long o4 = k > 0 ? -sz : 0, o5 = k < op.nz - 1 ? sz : 0;
+    float2 u[NB][7];
+    if (in) {
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const float2* xb = x + (long long)min(g + G * q, nrhs - 1) * ld + n;
+            u[q][0] = __ldg(xb + o0), u[q][1] = __ldg(xb + o1), u[q][2] = __ldg(xb + o2);
+            u[q][3] = __ldg(xb + o3), u[q][4] = __ldg(xb + o4), u[q][5] = __ldg(xb + o5);
+            u[q][6] = __ldg(xb);
+        }
+    }
+    __syncthreads();  // the barrier is initialised
+    // a copy that does not land within the bound (never seen): its rows are read
+    // directly, after a second bounded wait for it
+    const bool landed = mbar_wait(&bar, 0) || mbar_wait(&bar, 0);
+    if (!in) return;
+    const float4* c = landed ? rows[row] + 3 * threadIdx.x : op.cf + 3 * n;
+    const float4 c01 = c[0], c23 = c[1], c45 = c[2];
 #pragma unroll
     for (int q = 0; q < NB; ++q) {
         const int b = g + G * q;
         if (b < nrhs) {
-            const float2* xb = x + b * ld + n;
-            float2 v = __ldg(xb);
-            const float2 u0 = __ldg(xb + o0), u1 = __ldg(xb + o1), u2 = __ldg(xb + o2);
-            const float2 u3 = __ldg(xb + o3), u4 = __ldg(xb + o4), u5 = __ldg(xb + o5);
-            auto mac = [&](float cr, float ci, float2 u) {
-                v.x = fmaf(cr, u.x, fmaf(-ci, u.y, v.x));
-                v.y = fmaf(cr, u.y, fmaf(ci, u.x, v.y));
+            float2 v = u[q][6];
+            auto mac = [&](float cr, float ci, float2 w) {
+                v.x = fmaf(cr, w.x, fmaf(-ci, w.y, v.x));
+                v.y = fmaf(cr, w.y, fmaf(ci, w.x, v.y));
             };
-            mac(c01.x, c01.y, u0);
-            mac(c01.z, c01.w, u1);
-            mac(c23.x, c23.y, u2);
-            mac(c23.z, c23.w, u3);
-            mac(c45.x, c45.y, u4);
-            mac(c45.z, c45.w, u5);
+            mac(c01.x, c01.y, u[q][0]);
+            mac(c01.z, c01.w, u[q][1]);
+            mac(c23.x, c23.y, u[q][2]);
+            mac(c23.z, c23.w, u[q][3]);
+            mac(c45.x, c45.y, u[q][4]);
+            mac(c45.z, c45.w, u[q][5]);
             y[b * ld + n] = v;
         }
     }
@@ -702,13 +730,13 @@ int usv_operator_apply_kernel(const usv_scene* scene, const void* op_buf, int va
                     const float2* xf = (const float2*)x;
                     float2* yf = (float2*)y;
                     const int r = nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : nrhs <= 4 ? 4 : 8;
-                    const int rows = 8 / (r == 1 ? 1 : r / 2);  // rows of a CTA: 8 / groups
+                    const int rows = r == 8 ? 4 : 8;  // rows of a CTA: 8 / groups
                     const dim3 g3((s.nx + 31) / 32, (s.ny + rows - 1) / rows, s.nz);
                     const dim3 b3(32, 8);
                     if (r == 1) k_apply_kc_rhs<1, 1><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
                     else if (r == 2) k_apply_kc_rhs<2, 2><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
-                    else if (r == 4) k_apply_kc_rhs<4, 2><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
-                    else k_apply_kc_rhs<8, 2><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
+                    else if (r == 4) k_apply_kc_rhs<4, 4><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
+                    else k_apply_kc_rhs<8, 4><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
                 } else {
                     k_apply_kc<<<dim3(grid.x), 256, 0, strm>>>(v, (const float2*)x, (float2*)y, ld,
                                                                step, nrhs);
