@@ -715,10 +715,14 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
 template <typename R, typename S, bool MS>
 cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePlan& plan) {
     plan = CyclePlan{};
-    const int ctas = sms < kCycMaxCtas ? sms : kCycMaxCtas;
+    int ctas = sms < kCycMaxCtas ? sms : kCycMaxCtas;
     if (nrhs > ctas) return cudaSuccess;
     long long total = 0, before = 0, most = 0;
     for (int b = 0; b < nrhs; ++b) total += sizes[b];
+    // at least 256 nodes per CTA: with fewer the meetings of the extra CTAs cost
+    // more than their share of the work saves (24^3, 148 -> 54 CTAs: complex64
+    // 12.6 -> 12.2 us per step, bfloat16 11.8 -> 11.4, complex128 14.2 -> 13.1)
+    if (total / 256 < ctas) ctas = total / 256 > nrhs ? int(total / 256) : nrhs;
     const int spare = ctas - nrhs;
     for (int b = 0; b < nrhs; ++b) {  // the split of k_cycle
         const int share = 1 + int(spare * (before + sizes[b]) / total) - int(spare * before / total);

@@ -138,7 +138,7 @@ __device__ __forceinline__ double reduce_slot0(const GState& g, int b, double* s
 template <bool ADJ, typename C2, bool MS = false>
 __global__ void __launch_bounds__(256) k_residual(OpView<double> op, const double2* rhs,
                                                   const double2* x, long long ld, C2* V,
-                                                  GState g, int first, Step step) {
+                                                  GState g, int first, Step step, int sub) {
     const int b = blockIdx.y;
     if (g.kr > 0) first = !g.started[b];
     if (!first && (g.status[b] != ST_ACTIVE)) return;
@@ -149,6 +149,12 @@ __global__ void __launch_bounds__(256) k_residual(OpView<double> op, const doubl
         step = sl.step;
         nchunk = sl.nchunk;
     }
+    // sub > 1 (small grids): chunks of 2048 / sub nodes, so that a thread does
+    // not walk eight nodes one after the other while most SMs are idle; the
+    // partial sums then lie next to each other (sub <= g.ps)
+    nchunk *= sub;
+    const int chunk = g.chunk / sub;
+    const int pst = sub > 1 ? 1 : g.ps;
     const int ncta = rhs_ctas<MS>(g, b);
     if (int(blockIdx.x) >= ncta) return;
     __shared__ double sh[32];
@@ -158,8 +164,8 @@ __global__ void __launch_bounds__(256) k_residual(OpView<double> op, const doubl
     C2* v0 = cb.V + (long long)cb.kc * g.nv;
     double acc = 0.0, acc_s = 0.0;
     for (int ch = blockIdx.x; ch < nchunk; ch += ncta) {
-        const long long n0 = (long long)ch * g.chunk;
-        const long long n1 = min(n0 + g.chunk, op.n);
+        const long long n0 = (long long)ch * chunk;
+        const long long n1 = min(n0 + chunk, op.n);
         Node p = decode(n0 + threadIdx.x, op.nx, op.ny);
         for (long long n = n0 + threadIdx.x; n < n1; n += blockDim.x) {
             double2 r = rb[n];
@@ -177,18 +183,19 @@ __global__ void __launch_bounds__(256) k_residual(OpView<double> op, const doubl
     }
     acc = block_sum(acc, sh);
     acc_s = block_sum(acc_s, sh);
-    if (threadIdx.x == 0)
-        g.partial[((long long)b * g.nblk + blockIdx.x) * g.ps] = make_double2(acc, acc_s);
+    double2* part = g.partial + (long long)b * g.nblk * g.ps;
+    if (threadIdx.x == 0) part[(long long)blockIdx.x * pst] = make_double2(acc, acc_s);
     if (!last_block_done(&g.counter[b], ncta)) return;
     // FP64 norm of the residual (the convergence test, like the final gate)
     // and of its stored copy (the scale of the cycle's first basis vector)
-    const double t = reduce_slot0(g, b, sh, ncta);
-    double ts = 0.0;
-    {
-        const double2* pp = g.partial + (long long)b * g.nblk * g.ps;
-        for (int q = threadIdx.x; q < ncta; q += blockDim.x) ts += ld_cg(pp + (long long)q * g.ps).y;
-        ts = block_sum(ts, sh);
+    double t = 0.0, ts = 0.0;
+    for (int q = threadIdx.x; q < ncta; q += blockDim.x) {
+        const double2 v = ld_cg(part + (long long)q * pst);
+        t += v.x;
+        ts += v.y;
     }
+    t = block_sum(t, sh);
+    ts = block_sum(ts, sh);
     __shared__ int st_sh;
     const int m = g.m, kc = cb.kc;
     if (threadIdx.x == 0) {
@@ -2380,6 +2387,11 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
     };
     dim3 grid_res, grid_dots, grid_orth, grid_upd, grid_gates;
     if (int e = grid_for((const void*)k_residual<ADJ, C2, MS>, 256, 0, grid_res)) return e;
+    // Grids that do not fill the GPU with 2048-node CTAs (four per SM): quarters
+    // of a chunk (48^3, complex64: 26.5 -> 14.4 us per cycle; 64^3: 28.6 -> 22.3).
+    const bool small_grid = !p.max_ctas && (long long)B * g.nchunk <= 4LL * sms;
+    const int res_sub = small_grid && g.ps >= 4 ? 4 : 1;
+    if (res_sub > 1) grid_res.x = unsigned(g.nchunk * res_sub);
     // Arnoldi stencil + dots: per-warp dot tasks with direct loads (two
     // bulk-copy layouts measured slower at 128^3, see the dots kernel)
     const void* fn_dots = (const void*)k_dots<R, S, ADJ, kDotsThreads, MS>;
@@ -2510,7 +2522,7 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
     }
     USV_CUDA_TRY(cudaMemset2DAsync(x, ld * sizeof(double2), 0, g.n * sizeof(double2), B, strm));
     if (kr == 0) {
-        k_residual<ADJ, C2, MS><<<grid_res, 256, 0, strm>>>(op64, rhs, x, ld, V, g, 1, step);
+        k_residual<ADJ, C2, MS><<<grid_res, 256, 0, strm>>>(op64, rhs, x, ld, V, g, 1, step, res_sub);
         USV_CUDA_TRY(cudaGetLastError());
     }
     // Recycling: pinned host blocks for the per-cycle read of the Hessenberg /
@@ -2582,7 +2594,7 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
             fam_shared.push_back(0.0);
             fam_step.push_back(-1);
             fam_need.push_back(2);
-            k_residual<ADJ, C2, MS><<<grid_res, 256, 0, st>>>(op64, rhs, x, ld, V, g, 0, step);
+            k_residual<ADJ, C2, MS><<<grid_res, 256, 0, st>>>(op64, rhs, x, ld, V, g, 0, step, res_sub);
             USV_CUDA_TRY(mark(st, k++, capturing));
             fam.push_back(4);
             // per RHS: x, b, the stored residual; per launch: node record (R),
@@ -2664,7 +2676,7 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
             fam_need.push_back(3);
             USV_CUDA_TRY(cudaMemcpyAsync(hb_pin.p, ws + L.hb, hb_bytes, cudaMemcpyDeviceToHost, st));
         } else {
-            k_residual<ADJ, C2, MS><<<grid_res, 256, 0, st>>>(op64, rhs, x, ld, V, g, 0, step);
+            k_residual<ADJ, C2, MS><<<grid_res, 256, 0, st>>>(op64, rhs, x, ld, V, g, 0, step, res_sub);
             USV_CUDA_TRY(mark(st, k++, capturing));
             fam.push_back(4);
             // per RHS: x, b, the stored residual; per launch: node record (R),
