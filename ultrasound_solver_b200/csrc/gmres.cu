@@ -457,7 +457,10 @@ template <> struct LaneLoad<bf2> {
 template <> struct LaneLoad<float2> {
     static constexpr int NL = 2;
     float4 r;
-    __device__ __forceinline__ void load(const float2* p) { r = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void load(const float2* p, unsigned long long pol) {
+        const uint4 v = ld16(p, pol);
+        r = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+    }
     __device__ __forceinline__ void zero() { r = make_float4(0.f, 0.f, 0.f, 0.f); }
     __device__ __forceinline__ double2 get(int i) const {  // scaled by 2^-896
         return i ? make_double2(widen_scaled(__float_as_uint(r.z)), widen_scaled(__float_as_uint(r.w)))
@@ -470,7 +473,10 @@ template <> struct LaneLoad<double2> {
     // 123.0 -> 118.8 us per launch)
     static constexpr int NL = 1;
     double2 a;
-    __device__ __forceinline__ void load(const double2* p) { a = *p; }
+    __device__ __forceinline__ void load(const double2* p, unsigned long long pol) {
+        const uint4 v = ld16(p, pol);
+        a = *reinterpret_cast<const double2*>(&v);
+    }
     __device__ __forceinline__ void zero() { a = make_double2(0.0, 0.0); }
     __device__ __forceinline__ double2 get(int) const { return a; }
 };
@@ -519,6 +525,12 @@ __device__ __forceinline__ void dots_finish(GState& g, int b, int j, bool proj, 
         }
     }
     if (threadIdx.x == 0) g.counter[b] = 0;
+}
+
+// Chunks of DC nodes (of every right-hand side) whose j + 2 vectors fill the
+// share of L2 that a pass leaves to the next one.
+template <typename C2, int DC> __device__ __forceinline__ int l2_chunks(const GState& g, int j) {
+    return int(g.l2_keep / ((long long)(j + 2) * DC * int(sizeof(C2)) * gridDim.y));
 }
 
 // Arnoldi step j, part 1: each CTA computes its chunk of w = sigma_j K u_j
@@ -588,9 +600,12 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
     for (int task = threadIdx.x; task < tasks_t * segs; task += NT)
         segsum[task] = make_double2(0.0, 0.0);
     const int nphase = int((N + DC - 1) / DC);
+    const int keep_from = nphase - l2_chunks<C2, DC>(g, j);
     for (int ch = blockIdx.x, par = 0; ch < nphase; ch += ncta, par ^= NBUF - 1) {
         const long long n0 = (long long)ch * DC;
         const int len = int(min((long long)DC, N - n0));
+        // the chunks read last stay for the orthogonalisation, which starts there
+        const unsigned long long pol = ch >= keep_from ? l2_evict_normal() : l2_evict_first();
         YS* ys = ys_buf[par];
         // single buffer: the previous chunk's dots are done with ys. Double
         // buffer: every warp passed the barrier below after its dots of the
@@ -661,7 +676,7 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
 #pragma unroll
                         for (int u = 0; u < kDotUnroll; ++u) {
                             const int q = qb + 32 * u;
-                            a[u] = q < q1 ? ut[q] : make_uint4(0u, 0u, 0u, 0u);
+                            a[u] = q < q1 ? ld16(ut + q, pol) : make_uint4(0u, 0u, 0u, 0u);
                         }
 #pragma unroll
                         for (int u = 0; u < kDotUnroll; ++u) {
@@ -690,7 +705,7 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
 #pragma unroll
                     for (int u = 0; u < kDotUnroll; ++u) {
                         const int q = qb + 32 * u;
-                        if (q < q1) a[u].load(ut + NL * q);
+                        if (q < q1) a[u].load(ut + NL * q, pol);
                         else a[u].zero();
                     }
 #pragma unroll
@@ -1036,10 +1051,14 @@ __global__ void __launch_bounds__(OrthBulk<S>::THREADS) k_orth_bulk(S* V, long l
         if (lane == 0) {
             int q = 0;
             bool ok = true;
+            const int keep = l2_chunks<C2, kChunk>(g, j);
             for (int i = 0; i < nmy && ok; ++i) {
                 const long long n0 = (nchunk - 1 - blockIdx.x - (long long)i * ncta) * kChunk;
                 const int len = int(min((long long)kChunk, N - n0));
                 const unsigned bytes = unsigned((size_t(len) * sizeof(C2) + 15) / 16 * 16);
+                // the chunks read last stay for the next dots pass, which starts there
+                const unsigned long long pol =
+                    n0 < (long long)keep * kChunk ? l2_evict_normal() : l2_evict_first();
                 for (int tt = 0; tt < tpc; ++tt, ++q) {
                     const int s = q & (P::STAGES - 1);
                     if (!mbar_wait(&empty[s], (unsigned(q >> P::LOG_STAGES) & 1u) ^ 1u)) {
@@ -1050,7 +1069,7 @@ __global__ void __launch_bounds__(OrthBulk<S>::THREADS) k_orth_bulk(S* V, long l
                                             : (tt - 1 < cb.kc ? cb.C : cb.V) +
                                                   (long long)(tt - 1) * g.nv + n0;
                     mbar_expect_tx(&full[s], bytes);
-                    bulk_g2s(ring + size_t(s) * P::TILE, src, bytes, &full[s]);
+                    bulk_g2s_hint(ring + size_t(s) * P::TILE, src, bytes, &full[s], pol);
                 }
             }
             if (!ok) {
@@ -2363,6 +2382,17 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
     int dev = 0, sms = 0;
     USV_CUDA_TRY(cudaGetDevice(&dev));
     USV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // The dots and the orthogonalisation walk the basis in opposite directions;
+    // what a pass reads last is kept for the next one, the rest and the row
+    // coefficients go first. Two fifths of the L2 (50 of 126 MB: each half of
+    // the chip caches what its own SMs read) was the best share of 0, 30, 50,
+    // 70, 90 and 110 MB. Without hints / with: 62.3 / 56.8 ms (8 cycles of GCRO-DR(32,8),
+    // bfloat16, 128^3, 4 right-hand sides), 13.6 / 12.6 ms (GMRES(30), complex64,
+    // 128^3), 12.2 / 11.5 ms (complex128, 97 x 90 x 83, 2 right-hand sides; hints
+    // on its per-thread orthogonalisation loads cost 25 us per launch).
+    int l2 = 0;
+    USV_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+    g.l2_keep = (long long)l2 * 2 / 5;
     auto grid_for = [&](const void* fn, int threads, size_t smem, dim3& grid,
                         int fixed_per_sm = 0) -> int {
         int per_sm = fixed_per_sm;

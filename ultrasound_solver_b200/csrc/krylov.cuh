@@ -77,6 +77,7 @@ struct GState {
     ulonglong2* cyc_tot;   // [B][2 (m + 2)] totals (last entry: the norm)
     unsigned long long* cyc_flag;   // [ctas] step whose vector a CTA has stored
     unsigned long long* cyc_epoch;  // step number before the next launch
+    long long l2_keep; // bytes of a basis pass that the next pass is to find in L2
     const struct SceneSlot* slots;  // [B] multi-scene solves: the scene of each RHS
 };
 

@@ -144,6 +144,39 @@ __device__ __forceinline__ void bf_sq(float& rr, float& ii, unsigned y) {
         : "r"(y));
 }
 
+// ---------------------------------------------------------------- L2 policies
+// Eviction policy of loads (cache hints): lines read for the last time before
+// they would be evicted anyway go first, so that lines about to be read again
+// survive.
+__device__ __forceinline__ unsigned long long l2_evict_first() {
+    unsigned long long p;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ unsigned long long l2_evict_normal() {
+    unsigned long long p;
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint4 ld16(const void* p, unsigned long long policy) {
+    uint4 v;
+    asm volatile("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p), "l"(policy));
+    return v;
+}
+__device__ __forceinline__ uint2 ldg8(const void* p, unsigned long long policy) {
+    uint2 v;
+    asm("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(p), "l"(policy));
+    return v;
+}
+__device__ __forceinline__ float4 ldg16(const void* p, unsigned long long policy) {
+    float4 v;
+    asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(p), "l"(policy));
+    return v;
+}
 // ---------------------------------------------------------------- layout
 // Byte offsets of the operator buffer. Everything is derived from the scene,
 // so host and device agree without storing the layout itself.
@@ -395,7 +428,8 @@ template <typename S>
 __device__ __forceinline__ float2 k_row_cf(const OpView<float>& op, const S* __restrict__ u,
                                            long long n, Node p) {
     const float4* c = op.cf + 3 * n;
-    const float4 c01 = __ldg(c), c23 = __ldg(c + 1), c45 = __ldg(c + 2);
+    const unsigned long long pol = l2_evict_first();
+    const float4 c01 = ldg16(c, pol), c23 = ldg16(c + 1, pol), c45 = ldg16(c + 2, pol);
     const long long sy = op.nx, sz = (long long)op.nx * op.ny;
     const float2 u0 = widen<float2>(u[p.i > 0 ? n - 1 : n]);
     const float2 u1 = widen<float2>(u[p.i < op.nx - 1 ? n + 1 : n]);
@@ -425,7 +459,8 @@ template <typename S>
 __device__ __forceinline__ float2 k_row_cf_clamped(const OpView<float>& op,
                                                    const S* __restrict__ u, long long n) {
     const float4* c = op.cf + 3 * n;
-    const float4 c01 = __ldg(c), c23 = __ldg(c + 1), c45 = __ldg(c + 2);
+    const unsigned long long pol = l2_evict_first();
+    const float4 c01 = ldg16(c, pol), c23 = ldg16(c + 1, pol), c45 = ldg16(c + 2, pol);
     const long long sy = op.nx, sz = (long long)op.nx * op.ny, last = op.n - 1;
     const float2 u0 = widen<float2>(u[n > 0 ? n - 1 : 0]);
     const float2 u1 = widen<float2>(u[n < last ? n + 1 : last]);
@@ -453,7 +488,8 @@ __device__ __forceinline__ float2 k_row_cf_clamped(const OpView<float>& op,
 __device__ __forceinline__ float2 k_row_cb_clamped(const OpView<float>& op,
                                                    const bf2* __restrict__ u, long long n) {
     const uint2* c = op.cb + 3 * n;
-    const uint2 c01 = __ldg(c), c23 = __ldg(c + 1), c45 = __ldg(c + 2);
+    const unsigned long long pol = l2_evict_first();
+    const uint2 c01 = ldg8(c, pol), c23 = ldg8(c + 1, pol), c45 = ldg8(c + 2, pol);
     const long long sy = op.nx, sz = (long long)op.nx * op.ny, last = op.n - 1;
     const unsigned* w = reinterpret_cast<const unsigned*>(u);
     const unsigned u0 = w[n > 0 ? n - 1 : 0], u1 = w[n < last ? n + 1 : last];
@@ -722,6 +758,14 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
         ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, unsigned bytes, unsigned long long* bar,
+                                              unsigned long long policy) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+        ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
         : "memory");
 }
 
