@@ -194,3 +194,53 @@ def test_target_response_points_outside_the_grid():
                 row = (lo[0] + ci) + nx * ((lo[1] + cj) + ny * (lo[2] + ck))
                 acc += w * G[:, row]
     assert rel(got[0], acc) <= 1e-13
+
+
+@pytest.mark.parametrize("n,m", [(5000, 3), (262144, 5), (262145, 9), (900001, 4)])
+@pytest.mark.parametrize("precision", ["complex64", "complex128"])
+def test_basis_adjoint_forms(n, m, precision):
+    """Chunk length (2048 / 8192 nodes) and columns per CTA (1 / 4) by size, and
+    the workspace of the longer chunk: FP64 sums in another order, so 1e-12."""
+    from ultrasound_solver_b200 import _native as N
+    import ctypes as C
+    dtype = getattr(torch, precision)
+    prec = N.PREC_MIXED if precision == "complex64" else N.PREC_FP64
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    G = torch.randn(m, n, dtype=dtype, device="cuda", generator=gen)
+    g = torch.randn(n, dtype=torch.complex128, device="cuda", generator=gen)
+    ph = torch.rand(m, dtype=torch.float64, device="cuda", generator=gen)
+    want = G.to(torch.complex128).conj() @ g
+    nbytes = C.c_size_t()
+    N.check(N.load().usv_basis_adjoint_workspace_bytes(n, m, C.byref(nbytes)))
+    for size in (nbytes.value, 16 * m * ((n + 8191) // 8192)):
+        ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+        resp = torch.empty(m, dtype=torch.complex128, device="cuda")
+        N.check(N.load().usv_basis_adjoint(N.ptr(G), n, m, prec, N.ptr(g), N.ptr(ph), N.ptr(resp), None,
+                                           N.ptr(ws), size, N.stream_handle(torch, G.device)))
+        assert float((resp - want).abs().max() / want.abs().max()) < 1e-12
+
+
+def test_loss_many_targets():
+    """More targets than the fused launch adds (64), repeats among them."""
+    from ultrasound_solver_b200 import _native as N
+    import ctypes as C
+    n, nt = 10000, 100
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    u = torch.randn(n, dtype=torch.complex128, device="cuda", generator=gen)
+    idx = torch.randint(0, n, (nt,), device="cuda", generator=gen)
+    idx[1] = idx[0]
+    nbytes = C.c_size_t()
+    N.check(N.load().usv_loss_workspace_bytes(n, C.byref(nbytes)))
+    ws = torch.empty(nbytes.value, dtype=torch.uint8, device="cuda")
+    for count in (nt, 64, 3):
+        value = torch.empty(3, dtype=torch.float64, device="cuda")
+        cot = torch.empty_like(u)
+        N.check(N.load().usv_loss(N.LOSS_FOCAL_PRESSURE, N.ptr(u), n, None, N.ptr(idx), count, 1.5, 0.1, 1.0,
+                                  1e-12, N.ptr(value), N.ptr(cot), N.ptr(ws), nbytes.value,
+                                  N.stream_handle(torch, u.device)))
+        t = idx[:count]
+        want = u * (0.1 / n)
+        want.index_put_((t,), -1.5 / count * u[t] / (u[t].abs() + 1e-12), accumulate=True)
+        loss = -1.5 * u[t].abs().mean() + 0.05 * (u.abs() ** 2).mean()
+        assert abs(float(value[0] - loss)) < 1e-12
+        assert float((cot - want).abs().max()) < 1e-14

@@ -187,11 +187,11 @@ int usv_basis_adjoint(const void* basis, int64_t n, int m, int prec, const void*
                       size_t workspace_bytes, void* stream) {
     if (!basis || n < 1 || m < 1 || m > 65535 || !cotangent || !phases || !workspace)
         return USV_ERR_ARG;
-    size_t need = 0;
-    usv_basis_adjoint_workspace_bytes(n, m, &need);
-    if (workspace_bytes < need) return USV_ERR_WORKSPACE;
+    // (a workspace of the larger chunk's size is enough: then that chunk is used)
+    auto need = [&](long long c) { return sizeof(double2) * size_t((n + c - 1) / c) * size_t(m); };
+    if (workspace_bytes < need(kBasisChunk)) return USV_ERR_WORKSPACE;
     if (prec != USV_PREC_MIXED && prec != USV_PREC_FP64) return USV_ERR_ARG;
-    const int chunk = int(adjoint_chunk(n));
+    const int chunk = int(workspace_bytes < need(adjoint_chunk(n)) ? kBasisChunk : adjoint_chunk(n));
     const int nblk = int((n + chunk - 1) / chunk);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     double2* part = static_cast<double2*>(workspace);
