@@ -52,6 +52,7 @@ def _both(op, rhs, precision, **kw):
     ((64, 63, 61), 1, 30, 5, False),     # part of the basis read from global memory
     ((41, 40, 39), 4, 40, 3, False),     # more vector groups than warps hold at once
     ((24, 23, 22), 1, 100, 0, False),    # long basis
+    ((70, 69, 68), 1, 12, 3, False),     # 2240 nodes per CTA: the largest complex128 instance
     ((80, 79, 78), 1, 9, 4, True),       # 3392 nodes per CTA (complex128: per-pass kernels)
     ((90, 91, 89), 1, 11, 0, False),     # 4928 nodes per CTA: the largest instances
 ])

@@ -706,12 +706,14 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
 // The smallest instance whose CTAs hold the largest share of nodes a launch can
 // see: all right-hand sides active. Measured per Arnoldi step of GMRES(30),
 // this kernel / one launch per pass (us; nodes over all right-hand sides):
-//   bfloat16   14.0 / 29.4 at 14 k, 17.6 / 32.4 at 262 k, 24.4 / 38.4 at 593 k, 38.2 / 50.6 at 1.19 M,
-//              69.7 / 77.1 at 1.77 M, 85.4 / 88.3 at 2.10 M
-//   complex64  14.4 / 34.2         23.0 / 37.2            39.5 / 53.8          82.4 / 86.7
-//   complex128 14.8 / 40.7         31.8 / 48.8            102  / 85.9
-// so bfloat16 takes it up to 16384 nodes per CTA, complex64 up to 8192 and
-// complex128 up to 2048 (2.4 M, 1.2 M and 303 k nodes on 148 SMs).
+//   bfloat16   23.9 / 40.0 at 593 k, 34.2 / 49.6 at 1.00 M, 61.9 / 63.8 at 1.40 M, 71.8 / 73.1 at 1.73 M,
+//              72.7 / 72.5 at 1.82 M, 78.6 / 76.4 at 1.91 M, 84.3 / 78.7 at 2.10 M
+//   complex64  33.2 / 46.4 at 524 k, 60.4 / 65.1 at 729 k, 77.4 / 78.3 at 1.00 M, 72.8 / 72.8 at 1.05 M (4 x 64^3),
+//              84.3 / 80.0 at 1.12 M, 81.9 / 76.6 at 1.19 M
+//   complex128 30.2 / 50.8 at 262 k, 59.2 / 64.8 at 314 k, 61.7 / 67.0 at 365 k (4 x 45^3),
+//              68.2 / 68.2 at 373 k, 75.0 / 71.2 at 405 k
+// The two meet where the basis is far larger than L2 and both read it from
+// DRAM: 12288, 7104 and 2496 nodes per CTA (1.82 M, 1.05 M, 369 k on 148 SMs).
 template <typename R, typename S, bool MS>
 cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePlan& plan) {
     plan = CyclePlan{};
@@ -730,16 +732,16 @@ cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePl
         most = per > most ? per : most;
         before += sizes[b];
     }
+    constexpr int line = sizeof(S) == 4 ? 12288 : sizeof(S) == 8 ? 7104 : 2496;
     const void* fn = nullptr;
     int max_nodes = 0;
     auto take = [&](const void* f, int nodes) {
-        if (!fn && most <= nodes) fn = f, max_nodes = nodes;
+        if (!fn && most <= nodes && most <= line) fn = f, max_nodes = nodes;
     };
     constexpr int U0 = sizeof(S) == 16 ? 2 : 1;  // 2048, 1024, 1024 nodes per CTA and up
     take(reinterpret_cast<const void*>(k_cycle<R, S, MS, U0>), Geo<S, U0>::MAX);
     take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 2 * U0>), Geo<S, 2 * U0>::MAX);
-    if constexpr (sizeof(S) != 16)
-        take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 4 * U0>), Geo<S, 4 * U0>::MAX);
+    take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 4 * U0>), Geo<S, 4 * U0>::MAX);
     if constexpr (sizeof(S) != 16)
         take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 8 * U0>), Geo<S, 8 * U0>::MAX);
     if (!fn) return cudaSuccess;
