@@ -23,7 +23,7 @@ LIBDIR = PKG / "_lib"
 LIBNAME = "libusv_b200.so"
 SOURCES = ("operator.cu", "gmres.cu", "cycle.cu", "scene.cu", "basis.cu", "losses.cu", "surface.cu",
            "dense.cpp")
-HEADERS = ("usv_internal.cuh", "krylov.cuh", "dense.h")
+HEADERS = tuple(sorted(p.name for p in CSRC.iterdir() if p.suffix in (".cuh", ".h")))
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
