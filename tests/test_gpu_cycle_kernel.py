@@ -105,3 +105,61 @@ def test_scenes_and_finished_columns(precision):
         a, b = got[0][i, :o.n], got[1][i, :o.n]
         err = float(torch.linalg.norm(a - b) / torch.linalg.norm(b))
         assert err <= TOL[precision], (i, err)
+
+
+def _solve_scenes(ops, rhs, cap, **kw):
+    """usv_gmres_solve_scenes with one right-hand side per scene, up to the iteration cap."""
+    import ctypes as C
+    from ultrasound_solver_b200 import _native as N
+    from ultrasound_solver_b200.iterative_solver import B200IterativeSolver
+    count = len(ops)
+    it = B200IterativeSolver(max_ctas=cap, **kw)
+    p = it.params()
+    p.history_capacity = 0
+    scenes = (N.Scene * count)(*[o.scene for o in ops])
+    bufs = (C.c_void_p * count)(*[o.buffer.data_ptr() for o in ops])
+    of = (C.c_int * count)(*range(count))
+    nbytes = C.c_size_t()
+    lib = N.load()
+    N.check(lib.usv_gmres_scenes_workspace_bytes(count, scenes, of, C.byref(p), count, C.byref(nbytes)))
+    ws = torch.empty(nbytes.value, dtype=torch.uint8, device="cuda")
+    x = torch.empty_like(rhs)
+    stats = (N.GmresStats * count)()
+    N.check(lib.usv_gmres_solve_scenes(count, scenes, bufs, of, C.byref(p), N.ptr(rhs), N.ptr(x), count,
+                                       rhs.shape[1], N.ptr(ws), nbytes.value, stats,
+                                       N.stream_handle(torch, x.device)))
+    return x, stats
+
+
+@pytest.mark.parametrize("finished", ["zero", "easy"])
+@pytest.mark.parametrize("precision,edges", [("bf16", (12, 42, 64, 64)), ("mixed", (10, 40, 35, 35)),
+                                             ("fp64", (10, 33, 28, 45))])
+def test_share_that_grows_when_a_scene_finishes(precision, edges, finished):
+    """Scenes whose largest range is that of an instance while all are active
+    and one group of 64 nodes more once the first has finished: before the
+    first cycle (zero right-hand side) or between cycles (at a hundred times
+    the frequency its Jacobi-scaled rows are near the identity). Bounds as above."""
+    from ultrasound_solver_b200 import _native as N
+    from ultrasound_solver_b200.scene import DeviceOperator
+    ops = [_operator((n, n, n), 40 + i) for i, n in enumerate(edges)]
+    if finished == "easy":
+        n = edges[0]
+        full = lambda v: torch.full((n ** 3,), v, dtype=torch.float64, device="cuda")
+        ops[0] = DeviceOperator((n, n, n), 1e-3, 2 * np.pi * 4e6, FACES, full(1.2), full(343.0),
+                                pml={"cells": 2, "strength": 2.0, "order": 2})
+    ld = max(o.n for o in ops)
+    rhs = torch.zeros((len(ops), ld), dtype=torch.complex128, device="cuda")
+    for i, o in enumerate(ops):
+        if i > 0 or finished == "easy":
+            rhs[i, :o.n] = _rhs(1, o.n, 60 + i)[0]
+    kw = dict(restart=14, recycle=4, maxiter=56, rtol=1e-4, backward_error_tol=1.0, precision=precision)
+    (x, st), (y, st2) = (_solve_scenes(ops, rhs, cap, **kw) for cap in (0, 1 << 20))
+    assert st[0].status == N.USV_OK and st[0].iterations <= 28
+    for i, o in enumerate(ops):
+        assert st[i].iterations == st2[i].iterations
+        if i > 0:
+            assert st[i].iterations >= 48  # (whole cycles up to the cap)
+        if i > 0 or finished == "easy":
+            a, b = x[i, :o.n], y[i, :o.n]
+            err = float(torch.linalg.norm(a - b) / torch.linalg.norm(b))
+            assert err <= TOL[precision], (i, err)

@@ -30,6 +30,8 @@
 // ends the right-hand side with ST_DEVICE_TIMEOUT.
 #include "cycle.cuh"
 
+#include <type_traits>
+
 namespace usv {
 
 namespace {
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
     // the same split from the status words, which only change between
     // launches or on a failed wait).
     if (threadIdx.x == 0) {
-        // (32-bit arithmetic: the host launches at most kCycMaxCtas * G::MAX nodes)
+        // (32-bit arithmetic: cycle_shape takes at most kCycMaxCtas * cycle_line nodes)
         unsigned total = 0, active = 0;
 #pragma unroll 1
         for (int b = 0; b < nrhs; ++b)
@@ -327,15 +329,14 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
         who[0] = -1;
         who[3] = 0;
         unsigned before = 0, seen = 0;
-        const unsigned spare = gridDim.x - active;  // one CTA each, the rest by size
 #pragma unroll 1
         for (int b = 0; b < nrhs; ++b)
             if (g.status[b] == ST_ACTIVE) {
                 const unsigned own = MS ? unsigned(g.slots[b].n) : 1u;
-                const unsigned first = seen + unsigned((unsigned long long)spare * before / total);
+                const unsigned first = cycle_first_cta(gridDim.x, active, seen, before, total);
                 before += own;
                 ++seen;
-                const unsigned end = seen + unsigned((unsigned long long)spare * before / total);
+                const unsigned end = cycle_first_cta(gridDim.x, active, seen, before, total);
                 if (blockIdx.x >= first && blockIdx.x < end) {
                     who[0] = b;
                     who[1] = int(blockIdx.x - first);
@@ -350,10 +351,19 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
     if constexpr (MS) op = slot_view<R>(g.slots[b]);
     const CycleBasis<S> cb = cycle_basis(V, g, b);
     const int kc = cb.kc;
-    // node range of this CTA: whole 64-node groups (a vector's padding), at
-    // most G::MAX nodes (the host launches no other case)
+    // node range of this CTA: at most G::MAX nodes in every launch of a solve
+    // (cycle_shape). More would leave nodes out: such a right-hand side ends
+    // with an error, set by the least-squares kernel so that the status words
+    // do not change while other CTAs derive their split from them.
     const int N = int(op.n);
-    const int per = ((N + 63) / 64 + ncta - 1) / ncta * 64;
+    const int per = cycle_cta_nodes(N, ncta);
+    if (per > G::MAX) {
+        if (rank == 0 && threadIdx.x == 0) {
+            g.len[b] = -1;
+            g.ended[b] = 1;
+        }
+        return;
+    }
     const int lo = min(N, rank * per), len = min(N, lo + per) - lo;
     const int units = (len + NL - 1) / NL;
 
@@ -703,47 +713,28 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
     }
 }
 
-// The smallest instance whose CTAs hold the largest share of nodes a launch can
-// see: all right-hand sides active. Measured per Arnoldi step of GMRES(30),
-// this kernel / one launch per pass (us; nodes over all right-hand sides):
-//   bfloat16   23.9 / 40.0 at 593 k, 34.2 / 49.6 at 1.00 M, 61.9 / 63.8 at 1.40 M, 71.8 / 73.1 at 1.73 M,
-//              72.7 / 72.5 at 1.82 M, 78.6 / 76.4 at 1.91 M, 84.3 / 78.7 at 2.10 M
-//   complex64  33.2 / 46.4 at 524 k, 60.4 / 65.1 at 729 k, 77.4 / 78.3 at 1.00 M, 72.8 / 72.8 at 1.05 M (4 x 64^3),
-//              84.3 / 80.0 at 1.12 M, 81.9 / 76.6 at 1.19 M
-//   complex128 30.2 / 50.8 at 262 k, 59.2 / 64.8 at 314 k, 61.7 / 67.0 at 365 k (4 x 45^3),
-//              68.2 / 68.2 at 373 k, 75.0 / 71.2 at 405 k
-// The two meet where the basis is far larger than L2 and both read it from
-// DRAM: 12288, 7104 and 2496 nodes per CTA (1.82 M, 1.05 M, 369 k on 148 SMs).
+// Launch of the instance that cycle_shape picks.
 template <typename R, typename S, bool MS>
 cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePlan& plan) {
     plan = CyclePlan{};
-    int ctas = sms < kCycMaxCtas ? sms : kCycMaxCtas;
-    if (nrhs > ctas) return cudaSuccess;
-    long long total = 0, before = 0, most = 0;
-    for (int b = 0; b < nrhs; ++b) total += sizes[b];
-    // at least 256 nodes per CTA: with fewer the meetings of the extra CTAs cost
-    // more than their share of the work saves (24^3, 148 -> 54 CTAs: complex64
-    // 12.6 -> 12.2 us per step, bfloat16 11.8 -> 11.4, complex128 14.2 -> 13.1)
-    if (total / 256 < ctas) ctas = total / 256 > nrhs ? int(total / 256) : nrhs;
-    const int spare = ctas - nrhs;
-    for (int b = 0; b < nrhs; ++b) {  // the split of k_cycle
-        const int share = 1 + int(spare * (before + sizes[b]) / total) - int(spare * before / total);
-        const long long per = (sizes[b] + 64LL * share - 1) / (64LL * share) * 64;
-        most = per > most ? per : most;
-        before += sizes[b];
-    }
-    constexpr int line = sizeof(S) == 4 ? 12288 : sizeof(S) == 8 ? 7104 : 2496;
+    constexpr int bytes = int(sizeof(S));
+    const CycleShape shape = cycle_shape(bytes, sizes, nrhs, sms);
+    if (!shape.ctas) return cudaSuccess;
     const void* fn = nullptr;
     int max_nodes = 0;
-    auto take = [&](const void* f, int nodes) {
-        if (!fn && most <= nodes && most <= line) fn = f, max_nodes = nodes;
+    auto instance = [&](auto index) {
+        constexpr int I = decltype(index)::value;
+        if constexpr (I < cycle_instances(bytes)) {
+            using G = Geo<S, cycle_units(bytes, I)>;
+            static_assert(G::MAX == cycle_capacity(bytes, I), "room of an instance");
+            if (shape.instance == I)
+                fn = reinterpret_cast<const void*>(k_cycle<R, S, MS, cycle_units(bytes, I)>), max_nodes = G::MAX;
+        }
     };
-    constexpr int U0 = sizeof(S) == 16 ? 2 : 1;  // 2048, 1024, 1024 nodes per CTA and up
-    take(reinterpret_cast<const void*>(k_cycle<R, S, MS, U0>), Geo<S, U0>::MAX);
-    take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 2 * U0>), Geo<S, 2 * U0>::MAX);
-    take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 4 * U0>), Geo<S, 4 * U0>::MAX);
-    if constexpr (sizeof(S) != 16)
-        take(reinterpret_cast<const void*>(k_cycle<R, S, MS, 8 * U0>), Geo<S, 8 * U0>::MAX);
+    instance(std::integral_constant<int, 0>());
+    instance(std::integral_constant<int, 1>());
+    instance(std::integral_constant<int, 2>());
+    instance(std::integral_constant<int, 3>());
     if (!fn) return cudaSuccess;
     const CycFixed<S> fix(m, max_nodes);
     const size_t smem = 225 * 1024;
@@ -754,7 +745,7 @@ cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePl
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kCycThreads, smem);
     if (e != cudaSuccess || per_sm < 1) return e;
     plan.fn = fn;
-    plan.ctas = ctas;
+    plan.ctas = shape.ctas;
     plan.smem = smem;
     return cudaSuccess;
 }

@@ -1,12 +1,10 @@
 // One restart cycle's Arnoldi steps in a single launch (cycle.cu).
 #pragma once
 
+#include "cycle_split.h"
 #include "krylov.cuh"
 
 namespace usv {
-
-constexpr int kCycThreads = 512;
-constexpr int kCycMaxCtas = 512;  // size of the partial-sum rows in the workspace
 
 // Launch geometry of the cycle kernel for right-hand sides of sizes[b] nodes;
 // ctas = 0: this solve keeps one launch per Arnoldi pass.

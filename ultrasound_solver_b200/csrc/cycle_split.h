@@ -1,0 +1,85 @@
+// How the CTAs of a cycle launch (cycle.cu) are shared out over the right-hand
+// sides, and which kernel instance holds every division a launch can see.
+// Plain C++: the kernel, its launcher and a host test use the same functions.
+#pragma once
+
+#ifdef __CUDACC__
+#define USV_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define USV_HOST_DEVICE inline
+#endif
+
+namespace usv {
+
+constexpr int kCycThreads = 512;
+constexpr int kCycMaxCtas = 512;  // size of the partial-sum rows in the workspace
+
+// Every active right-hand side gets one CTA, the other ctas - active go by size.
+// First CTA of the one that follows `seen` active right-hand sides of `before`
+// units, of `total` (nodes; 1 for each right-hand side of a single scene).
+USV_HOST_DEVICE unsigned cycle_first_cta(unsigned ctas, unsigned active, unsigned seen, unsigned before,
+                                         unsigned total) {
+    return seen + unsigned((unsigned long long)(ctas - active) * before / total);
+}
+
+// Nodes of one of `share` CTAs for n nodes: whole 64-node groups (a vector's padding).
+USV_HOST_DEVICE int cycle_cta_nodes(int n, int share) { return ((n + 63) / 64 + share - 1) / share * 64; }
+
+// Instances by bytes per stored value: nodes a CTA of instance i has room for.
+constexpr int cycle_instances(int bytes) { return bytes == 16 ? 3 : 4; }
+constexpr int cycle_units(int bytes, int i) { return (bytes == 16 ? 2 : 1) << i; }  // 16-byte loads per thread
+constexpr int cycle_capacity(int bytes, int i) { return kCycThreads * (16 / bytes) * cycle_units(bytes, i); }
+
+// Most nodes per CTA for which the cycle kernel is taken. Measured per Arnoldi
+// step of GMRES(30), cycle kernel / one launch per pass (us; nodes over all
+// right-hand sides):
+//   bfloat16   23.9 / 40.0 at 593 k, 34.2 / 49.6 at 1.00 M, 61.9 / 63.8 at 1.40 M, 71.8 / 73.1 at 1.73 M,
+//              72.7 / 72.5 at 1.82 M, 78.6 / 76.4 at 1.91 M, 84.3 / 78.7 at 2.10 M
+//   complex64  33.2 / 46.4 at 524 k, 60.4 / 65.1 at 729 k, 77.4 / 78.3 at 1.00 M, 72.8 / 72.8 at 1.05 M (4 x 64^3),
+//              84.3 / 80.0 at 1.12 M, 81.9 / 76.6 at 1.19 M
+//   complex128 30.2 / 50.8 at 262 k, 59.2 / 64.8 at 314 k, 61.7 / 67.0 at 365 k (4 x 45^3),
+//              68.2 / 68.2 at 373 k, 75.0 / 71.2 at 405 k
+// The two meet where the basis is far larger than L2 and both read it from
+// DRAM: 1.82 M, 1.05 M and 369 k nodes on 148 SMs.
+constexpr int cycle_line(int bytes) { return bytes == 4 ? 12288 : bytes == 8 ? 7104 : 2496; }
+
+struct CycleShape {
+    int ctas = 0;       // 0: one launch per Arnoldi pass
+    int instance = -1;
+};
+
+// Shape for right-hand sides of sizes[b] nodes on `sms` SMs: the smallest
+// instance that has room in every launch of the solve. Right-hand sides leave
+// as they finish. One that is still active then has at least the share
+// 1 + floor(spare n / total) formed here with all of them: `spare` only grows,
+// the active total only shrinks, and its real share is a difference of two
+// floors, at least the floor of the difference. (Its share in a particular
+// launch is no bound: a right-hand side rounded up there can be rounded down
+// once another has left. bfloat16 scenes of 12^3, 42^3, 64^3, 64^3 on 148 SMs:
+// 4096 nodes for the 42^3 one with all active, 4160 without the smallest.)
+inline CycleShape cycle_shape(int bytes, const long long* sizes, int nrhs, int sms) {
+    CycleShape shape;
+    int ctas = sms < kCycMaxCtas ? sms : kCycMaxCtas;
+    if (nrhs > ctas) return shape;
+    long long total = 0, most = 0;
+    for (int b = 0; b < nrhs; ++b) total += sizes[b];
+    if (total > (long long)ctas * cycle_line(bytes)) return shape;
+    // at least 256 nodes per CTA: with fewer the meetings of the extra CTAs cost
+    // more than their share of the work saves (24^3, 148 -> 54 CTAs: complex64
+    // 12.6 -> 12.2 us per step, bfloat16 11.8 -> 11.4, complex128 14.2 -> 13.1)
+    if (total / 256 < ctas) ctas = total / 256 > nrhs ? int(total / 256) : nrhs;
+    for (int b = 0; b < nrhs; ++b) {
+        const int per = cycle_cta_nodes(int(sizes[b]), 1 + int((long long)(ctas - nrhs) * sizes[b] / total));
+        most = per > most ? per : most;
+    }
+    if (most > cycle_line(bytes)) return shape;
+    for (int i = 0; i < cycle_instances(bytes); ++i)
+        if (most <= cycle_capacity(bytes, i)) {
+            shape.ctas = ctas;
+            shape.instance = i;
+            break;
+        }
+    return shape;
+}
+
+}  // namespace usv

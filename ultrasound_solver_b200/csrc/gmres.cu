@@ -1188,6 +1188,11 @@ __global__ void __launch_bounds__(128) k_lsq(GState g) {
     if (g.status[b] != ST_ACTIVE || !g.ended[b]) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int m = g.m, L = g.len[b];
+    if (RAW && L < 0) {  // refused by the cycle kernel
+        __syncthreads();  // (every thread has read the status)
+        if (threadIdx.x == 0) g.status[b] = ST_TOO_LARGE;
+        return;
+    }
     const int ldr = RAW ? L + 1 : L;
     double2* Rs = reinterpret_cast<double2*>(smem_raw);  // ldr x L, column-major
     double2* gv = Rs + (size_t)ldr * L;
@@ -2903,6 +2908,7 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
         st.info = (status[b] != ST_CONVERGED && iters[b] == p.maxiter) ? iters[b] : 0;
         const bool finite = gates[4 * b + 2] == 0.0;
         if (status[b] == ST_DEVICE_TIMEOUT) st.status = USV_ERR_DEVICE_TIMEOUT;
+        else if (status[b] == ST_TOO_LARGE) st.status = USV_ERR_TOO_LARGE;
         else if (!finite || status[b] == ST_NONFINITE) st.status = USV_ERR_NONFINITE;
         else if (st.info != 0 || status[b] != ST_CONVERGED || !(st.scaled_residual <= p.rtol) ||
                  !(st.backward_error <= p.backward_error_tol))

@@ -10,7 +10,8 @@
 namespace usv {
 
 enum { ST_ACTIVE = 0, ST_CONVERGED = 1, ST_MAXITER = 2, ST_NONFINITE = 3,
-       ST_DEVICE_TIMEOUT = 4 };  // a bounded device-side wait ran out
+       ST_DEVICE_TIMEOUT = 4,  // a bounded device-side wait ran out
+       ST_TOO_LARGE = 5 };     // more nodes per CTA than a kernel has room for
 
 // Per-RHS control words of a recycled (GCRO-DR) cycle, written by the host
 // before each cycle.
