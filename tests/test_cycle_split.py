@@ -42,6 +42,8 @@ extern "C" int most(const long long* sizes, const long long* units, const unsign
         }
     return last == unsigned(ctas) ? most : -1;
 }
+extern "C" int segments(int groups, int nodes) { return cycle_segments(groups, nodes); }
+extern "C" int task_room(int groups, int capacity) { return cycle_task_room(groups, capacity); }
 """
 
 
@@ -130,3 +132,18 @@ def test_room_for_one_scene(lib, nbytes):
             ctas, _ = _check(lib, nbytes, [n] * nrhs, [set(range(k)) for k in range(1, nrhs + 1)],
                              units=[1] * nrhs)
             assert ctas == 0 if nrhs > 148 else ctas >= 0
+
+
+@pytest.mark.parametrize("capacity", [1024, 2048, 4096, 8192, 16384])
+def test_room_for_the_sums_of_every_dots_task(lib, capacity):
+    """All restarts up to the largest (112: 28 groups of four vectors) and all
+    node counts of an instance; lane sums of at most 128 nodes."""
+    for restart in range(1, 113):
+        most = (restart + 3) // 4
+        room = lib.task_room(most, capacity)
+        for groups in {1, most // 2 or 1, most - 1 or 1, most}:
+            for nodes in {64, 4096, 4160, 8192, 8256, 12288, 12352, capacity - 64, capacity}:
+                if nodes <= capacity:
+                    segs = lib.segments(groups, nodes)
+                    assert groups * segs <= room
+                    assert -(-nodes // segs) <= 4096

@@ -163,3 +163,18 @@ def test_share_that_grows_when_a_scene_finishes(precision, edges, finished):
             a, b = x[i, :o.n], y[i, :o.n]
             err = float(torch.linalg.norm(a - b) / torch.linalg.norm(b))
             assert err <= TOL[precision], (i, err)
+
+
+@pytest.mark.parametrize("restart", [12, 100])
+def test_more_than_8192_nodes_per_cta(restart):
+    """The largest bfloat16 instance (three segments of nodes per CTA), with
+    more dots tasks than a short basis has (25 groups of vectors)."""
+    shape = (87, 86, 85)
+    ops = [_operator(shape, 70 + i) for i in range(2)]
+    rhs = torch.cat([_rhs(1, o.n, 80 + i) for i, o in enumerate(ops)])
+    kw = dict(restart=restart, maxiter=2 * restart, rtol=1e-13, precision="bf16")
+    (x, st), (y, st2) = (_solve_scenes(ops, rhs, cap, **kw) for cap in (0, 1 << 20))
+    for b in range(2):
+        assert st[b].iterations == st2[b].iterations
+        err = float(torch.linalg.norm(x[b] - y[b]) / torch.linalg.norm(y[b]))
+        assert err <= TOL["bf16"], (b, err)

@@ -37,7 +37,6 @@ namespace usv {
 namespace {
 
 constexpr int kCycWarps = kCycThreads / 32;
-constexpr int kCycTasks = 64;  // most dots tasks: vector groups x segments
 static_assert((USV_MAX_RESTART + 1 + kDotVecs) / kDotVecs <= 32, "group counts of the segment table");
 
 // UN 16-byte loads per thread and vector slice; NL nodes per load.
@@ -56,7 +55,8 @@ template <typename S> struct CycFixed {
     __host__ __device__ CycFixed(int m, int max_nodes) {
         auto up = [](size_t b) { return (b + 127) / 128 * 128; };
         dots = 0;
-        hs = up(sizeof(double) * 2 * kDotVecs * kCycTasks);
+        // (a step has at most m dots)
+        hs = up(sizeof(double) * 2 * kDotVecs * cycle_task_room((m + kDotVecs - 1) / kDotVecs, max_nodes));
         hm = hs + up(sizeof(double2) * (m + 2));
         sig = hm + up(sizeof(double2) * (m + 2));
         segs = sig + up(sizeof(double) * (m + 2));
@@ -395,19 +395,8 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
     ulonglong2* ntot = tot + 2 * (m + 1) + 1;
     unsigned long long epoch = *g.cyc_epoch;  // advanced between launches
 
-    // segments per vector group that balance the dots tasks over the warps
-    // (fewest vector slices per warp, then fewest segments)
-    if (threadIdx.x < 32) {
-        const int groups = threadIdx.x < 1 ? 1 : threadIdx.x;
-        const int least = (per + 4095) / 4096;  // at most 128 nodes per lane and segment
-        int best = least, rounds = (groups * least + kCycWarps - 1) / kCycWarps;  // rounds / best: slices per warp
-#pragma unroll 1
-        for (int sg = least + 1; groups * sg <= kCycTasks; ++sg) {
-            const int r = (groups * sg + kCycWarps - 1) / kCycWarps;
-            if (r * best < rounds * sg) best = sg, rounds = r;
-        }
-        seg_table[threadIdx.x] = best;
-    }
+    // segments per vector group
+    if (threadIdx.x < 32) seg_table[threadIdx.x] = cycle_segments(threadIdx.x < 1 ? 1 : threadIdx.x, per);
 #pragma unroll 1
     for (int t = threadIdx.x; t <= kc; t += NT) sig[t] = g.sigma[(long long)b * (m + 1) + t];
 #pragma unroll 1

@@ -25,6 +25,31 @@ USV_HOST_DEVICE unsigned cycle_first_cta(unsigned ctas, unsigned active, unsigne
 // Nodes of one of `share` CTAs for n nodes: whole 64-node groups (a vector's padding).
 USV_HOST_DEVICE int cycle_cta_nodes(int n, int share) { return ((n + 63) / 64 + share - 1) / share * 64; }
 
+// The dots of a step are (vector group, segment of the CTA's nodes) tasks, a warp
+// each. A segment holds at most 4096 nodes: 128 per lane, the longest fp32 sum
+// of a bfloat16 basis.
+constexpr int kCycTasks = 64;  // tasks that further segments may fill
+USV_HOST_DEVICE constexpr int cycle_least_segments(int nodes) { return (nodes + 4095) / 4096; }
+
+// Segments that balance the tasks of `groups` vector groups over the warps:
+// fewest vector slices per warp, then fewest segments.
+USV_HOST_DEVICE int cycle_segments(int groups, int nodes) {
+    constexpr int warps = kCycThreads / 32;
+    int best = cycle_least_segments(nodes), rounds = (groups * best + warps - 1) / warps;  // rounds / best: slices per warp
+#pragma unroll 1
+    for (int sg = best + 1; groups * sg <= kCycTasks; ++sg) {
+        const int r = (groups * sg + warps - 1) / warps;
+        if (r * best < rounds * sg) best = sg, rounds = r;
+    }
+    return best;
+}
+
+// Tasks whose sums need room in an instance of `capacity` nodes with at most
+// `groups` vector groups: the least segments of a long basis exceed kCycTasks.
+USV_HOST_DEVICE constexpr int cycle_task_room(int groups, int capacity) {
+    return groups * cycle_least_segments(capacity) > kCycTasks ? groups * cycle_least_segments(capacity) : kCycTasks;
+}
+
 // Instances by bytes per stored value: nodes a CTA of instance i has room for.
 constexpr int cycle_instances(int bytes) { return bytes == 16 ? 3 : 4; }
 constexpr int cycle_units(int bytes, int i) { return (bytes == 16 ? 2 : 1) << i; }  // 16-byte loads per thread
