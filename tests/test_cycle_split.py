@@ -15,8 +15,8 @@ from ultrasound_solver_b200 import build
 SOURCE = r"""
 #include "cycle_split.h"
 using namespace usv;
-extern "C" void shape(int bytes, const long long* sizes, int nrhs, int sms, int* ctas, int* room) {
-    const CycleShape s = cycle_shape(bytes, sizes, nrhs, sms);
+extern "C" void shape(int bytes, int scenes, const long long* sizes, int nrhs, int sms, int* ctas, int* room) {
+    const CycleShape s = cycle_shape(bytes, scenes != 0, sizes, nrhs, sms);
     *ctas = s.ctas;
     *room = s.ctas ? cycle_capacity(bytes, s.instance) : 0;
 }
@@ -66,7 +66,7 @@ def _array(values):
 def _check(lib, nbytes, sizes, subsets, sms=148, units=None):
     """Shape of the batch, after a look at the given subsets of it."""
     ctas, room = C.c_int(), C.c_int()
-    lib.shape(nbytes, _array(sizes), len(sizes), sms, C.byref(ctas), C.byref(room))
+    lib.shape(nbytes, 0 if units else 1, _array(sizes), len(sizes), sms, C.byref(ctas), C.byref(room))
     if ctas.value:
         for active in subsets:
             flags = bytes(1 if b in active else 0 for b in range(len(sizes)))
@@ -128,7 +128,7 @@ def test_room_for_one_scene(lib, nbytes):
     rng = random.Random(nbytes + 1)
     for nrhs in [1, 2, 3, 4, 7, 30, 147, 148, 149]:
         for _ in range(40):
-            n = rng.randint(8, 1_900_000 // nrhs)
+            n = rng.randint(8, 1_250_000 // nrhs)
             ctas, _ = _check(lib, nbytes, [n] * nrhs, [set(range(k)) for k in range(1, nrhs + 1)],
                              units=[1] * nrhs)
             assert ctas == 0 if nrhs > 148 else ctas >= 0
@@ -147,3 +147,16 @@ def test_room_for_the_sums_of_every_dots_task(lib, capacity):
                     segs = lib.segments(groups, nodes)
                     assert groups * segs <= room
                     assert -(-nodes // segs) <= 4096
+
+
+@pytest.mark.parametrize("nbytes,sizes,scenes,taken", [
+    (4, [104 ** 3], False, True), (4, [112 ** 3], False, False), (4, [74 ** 3] * 4, False, False),
+    (8, [84 ** 3], False, True), (8, [88 ** 3], False, False), (8, [60 ** 3] * 4, False, False),
+    (16, [66 ** 3], False, True), (16, [68 ** 3], False, False), (16, [43 ** 3] * 4, False, False),
+    (4, [48 ** 3, 80 ** 3, 64 ** 3] * 2, True, True), (4, [80 ** 3] * 4, True, False),
+    (8, [70 ** 3, 70 ** 3, 64 ** 3], True, True), (16, [45 ** 3] * 3 + [40 ** 3], True, False),
+])
+def test_cycle_kernel_only_where_overlapped_solves_keep_up(lib, nbytes, sizes, scenes, taken):
+    """Sizes at which solves on several streams were timed with and without it."""
+    ctas, _ = _check(lib, nbytes, sizes, [], units=None if scenes else [1] * len(sizes))
+    assert (ctas > 0) == taken

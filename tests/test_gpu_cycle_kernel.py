@@ -52,9 +52,9 @@ def _both(op, rhs, precision, **kw):
     ((64, 63, 61), 1, 30, 5, False),     # part of the basis read from global memory
     ((41, 40, 39), 4, 40, 3, False),     # more vector groups than warps hold at once
     ((24, 23, 22), 1, 100, 0, False),    # long basis
-    ((70, 69, 68), 1, 12, 3, False),     # 2240 nodes per CTA: the largest complex128 instance
-    ((80, 79, 78), 1, 9, 4, True),       # 3392 nodes per CTA (complex128: per-pass kernels)
-    ((90, 91, 89), 1, 11, 0, False),     # 4928 nodes per CTA: the largest instances
+    ((70, 69, 68), 1, 12, 3, False),     # 2240 nodes per CTA (complex128: both sides per-pass kernels)
+    ((80, 79, 78), 1, 9, 4, True),       # 3392 nodes per CTA (complex128: as above)
+    ((90, 91, 89), 1, 11, 0, False),     # 4928 nodes per CTA (bfloat16 only)
 ])
 def test_against_per_pass_kernels(precision, shape, nrhs, restart, recycle, adjoint):
     op = _operator(shape, 5)
@@ -178,3 +178,24 @@ def test_more_than_8192_nodes_per_cta(restart):
         assert st[b].iterations == st2[b].iterations
         err = float(torch.linalg.norm(x[b] - y[b]) / torch.linalg.norm(y[b]))
         assert err <= TOL["bf16"], (b, err)
+
+
+@pytest.mark.parametrize("precision,shape,scenes,recycle", [
+    ("bf16", (105, 106, 107), 1, 4),    # 8064 of 8192 nodes per CTA
+    ("mixed", (84, 84, 85), 1, 0),      # 4096 of 4096
+    ("fp64", (66, 65, 67), 1, 3),       # 1984 of 2048
+    ("mixed", (75, 76, 77), 2, 4),      # 5952 of 8192, scenes in one launch
+])
+def test_largest_instances(precision, shape, scenes, recycle):
+    """The instances with most nodes per CTA, near the sizes where they end. Bounds as above."""
+    ops = [_operator(shape, 90 + i) for i in range(scenes)]
+    rhs = torch.cat([_rhs(1, o.n, 95 + i) for i, o in enumerate(ops)])
+    kw = dict(restart=13, recycle=recycle, maxiter=39)
+    if scenes == 1:
+        (x, st), (y, st2) = _both(ops[0], rhs, precision, **kw)
+        assert st[0]["iterations"] == st2[0]["iterations"]
+    else:
+        (x, _), (y, _) = (_solve_scenes(ops, rhs, cap, rtol=1e-13, precision=precision, **kw) for cap in (0, 1 << 20))
+    for b in range(scenes):
+        err = float(torch.linalg.norm(x[b] - y[b]) / torch.linalg.norm(y[b]))
+        assert err <= TOL[precision], (b, err)

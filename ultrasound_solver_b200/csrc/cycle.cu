@@ -707,13 +707,13 @@ template <typename R, typename S, bool MS>
 cudaError_t cycle_plan(int m, const long long* sizes, int nrhs, int sms, CyclePlan& plan) {
     plan = CyclePlan{};
     constexpr int bytes = int(sizeof(S));
-    const CycleShape shape = cycle_shape(bytes, sizes, nrhs, sms);
+    const CycleShape shape = cycle_shape(bytes, MS, sizes, nrhs, sms);
     if (!shape.ctas) return cudaSuccess;
     const void* fn = nullptr;
     int max_nodes = 0;
     auto instance = [&](auto index) {
         constexpr int I = decltype(index)::value;
-        if constexpr (I < cycle_instances(bytes)) {
+        if constexpr (I < cycle_instances(bytes, MS)) {
             using G = Geo<S, cycle_units(bytes, I)>;
             static_assert(G::MAX == cycle_capacity(bytes, I), "room of an instance");
             if (shape.instance == I)

@@ -51,22 +51,36 @@ USV_HOST_DEVICE constexpr int cycle_task_room(int groups, int capacity) {
 }
 
 // Instances by bytes per stored value: nodes a CTA of instance i has room for.
-constexpr int cycle_instances(int bytes) { return bytes == 16 ? 3 : 4; }
+// (scenes: right-hand sides of several scenes in one launch)
+constexpr int cycle_instances(int bytes, bool scenes) { return bytes == 16 ? 2 : scenes ? 4 : 3; }
 constexpr int cycle_units(int bytes, int i) { return (bytes == 16 ? 2 : 1) << i; }  // 16-byte loads per thread
 constexpr int cycle_capacity(int bytes, int i) { return kCycThreads * (16 / bytes) * cycle_units(bytes, i); }
 
-// Most nodes per CTA for which the cycle kernel is taken. Measured per Arnoldi
-// step of GMRES(30), cycle kernel / one launch per pass (us; nodes over all
-// right-hand sides):
+// Most nodes per CTA for which the cycle kernel is taken. Alone it is the
+// faster one up to 12288, 7104 and 2496 nodes, per Arnoldi step of GMRES(30),
+// cycle kernel / one launch per pass (us; nodes over all right-hand sides):
 //   bfloat16   23.9 / 40.0 at 593 k, 34.2 / 49.6 at 1.00 M, 61.9 / 63.8 at 1.40 M, 71.8 / 73.1 at 1.73 M,
 //              72.7 / 72.5 at 1.82 M, 78.6 / 76.4 at 1.91 M, 84.3 / 78.7 at 2.10 M
 //   complex64  33.2 / 46.4 at 524 k, 60.4 / 65.1 at 729 k, 77.4 / 78.3 at 1.00 M, 72.8 / 72.8 at 1.05 M (4 x 64^3),
 //              84.3 / 80.0 at 1.12 M, 81.9 / 76.6 at 1.19 M
 //   complex128 30.2 / 50.8 at 262 k, 59.2 / 64.8 at 314 k, 61.7 / 67.0 at 365 k (4 x 45^3),
 //              68.2 / 68.2 at 373 k, 75.0 / 71.2 at 405 k
-// The two meet where the basis is far larger than L2 and both read it from
-// DRAM: 1.82 M, 1.05 M and 369 k nodes on 148 SMs.
-constexpr int cycle_line(int bytes) { return bytes == 4 ? 12288 : bytes == 8 ? 7104 : 2496; }
+// where the basis is far larger than L2 and both read it from DRAM. But its
+// launches hold the shared memory of their SMs, so those of solves on other
+// streams wait, while per-pass kernels overlap. Solves at once, each on its own
+// stream, ms (2 / 8 solves):
+//   bfloat16   104^3 22.4 / 88 against 23.1 / 93, 112^3 34.6 / 141 against 28.7 / 123 (GMRES(30)),
+//              104^3 40.2 / 161 against 40.4 / 163, 112^3 62.6 / 253 against 49.6 / 198 (GCRO-DR(36,8))
+//   complex64  84^3 22.8 / 90 against 23.0 / 97, 88^3 32.6 / 129 against 27.3 / 119
+//   complex128 66^3 18.8 / 77 against 23.2 / 95, 68^3 34.0 / 137 against 27.4 / 115
+// So one scene goes as far as it wins both ways: 8192, 4096 and 2048 nodes. A
+// batch of scenes is itself the overlap; two batches at once (100 iterations)
+// took 25.4 ms against 25.1 (bfloat16, 1.59 M nodes), 17.4 against 20.4
+// (complex64, 948 k), and 13.3 against 11.9 (complex128, 337 k), so the first
+// two go on to where the kernels meet alone.
+constexpr int cycle_line(int bytes, bool scenes) {
+    return bytes == 4 ? (scenes ? 12288 : 8192) : bytes == 8 ? (scenes ? 7104 : 4096) : 2048;
+}
 
 struct CycleShape {
     int ctas = 0;       // 0: one launch per Arnoldi pass
@@ -82,13 +96,14 @@ struct CycleShape {
 // launch is no bound: a right-hand side rounded up there can be rounded down
 // once another has left. bfloat16 scenes of 12^3, 42^3, 64^3, 64^3 on 148 SMs:
 // 4096 nodes for the 42^3 one with all active, 4160 without the smallest.)
-inline CycleShape cycle_shape(int bytes, const long long* sizes, int nrhs, int sms) {
+inline CycleShape cycle_shape(int bytes, bool scenes, const long long* sizes, int nrhs, int sms) {
+    const int line = cycle_line(bytes, scenes);
     CycleShape shape;
     int ctas = sms < kCycMaxCtas ? sms : kCycMaxCtas;
     if (nrhs > ctas) return shape;
     long long total = 0, most = 0;
     for (int b = 0; b < nrhs; ++b) total += sizes[b];
-    if (total > (long long)ctas * cycle_line(bytes)) return shape;
+    if (total > (long long)ctas * line) return shape;
     // at least 256 nodes per CTA: with fewer the meetings of the extra CTAs cost
     // more than their share of the work saves (24^3, 148 -> 54 CTAs: complex64
     // 12.6 -> 12.2 us per step, bfloat16 11.8 -> 11.4, complex128 14.2 -> 13.1)
@@ -97,8 +112,8 @@ inline CycleShape cycle_shape(int bytes, const long long* sizes, int nrhs, int s
         const int per = cycle_cta_nodes(int(sizes[b]), 1 + int((long long)(ctas - nrhs) * sizes[b] / total));
         most = per > most ? per : most;
     }
-    if (most > cycle_line(bytes)) return shape;
-    for (int i = 0; i < cycle_instances(bytes); ++i)
+    if (most > line) return shape;
+    for (int i = 0; i < cycle_instances(bytes, scenes); ++i)
         if (most <= cycle_capacity(bytes, i)) {
             shape.ctas = ctas;
             shape.instance = i;
