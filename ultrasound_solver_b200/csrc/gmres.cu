@@ -24,18 +24,16 @@
 // Basis vectors are stored unnormalised with a scale sigma_t = 1/||u_t||.
 #include <algorithm>
 #include <cmath>
-#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <type_traits>
 #include <vector>
 
 #include "cycle.cuh"
 #include "dense.h"
+#include "host_pool.h"
 
 static_assert(sizeof(usv_gmres_params) == 80, "usv_gmres_params layout (include/usv.h)");
 
@@ -2279,83 +2277,6 @@ static bool recycle_coefficients(int m, int k, const double* hb, std::vector<dou
     }
     return finite;
 }
-
-// Host threads of one solve for the harmonic Ritz steps of its right-hand
-// sides: on small grids a cycle takes less GPU time (0.4 ms) than the steps of
-// a few right-hand sides one after the other (0.3-0.5 ms each). Started with
-// the solve and joined when it returns; a solve of one right-hand side has none.
-class HostPool {
-  public:
-    explicit HostPool(int helpers) {
-        try {
-            for (int i = 0; i < helpers; ++i) threads_.emplace_back([this] { work(); });
-        } catch (const std::system_error&) {  // fewer threads, or none: the caller works too
-        }
-    }
-    ~HostPool() {
-        {
-            std::lock_guard<std::mutex> l(lock_);
-            stop_ = true;
-        }
-        start_.notify_all();
-        for (auto& t : threads_) t.join();
-    }
-    HostPool(const HostPool&) = delete;
-    HostPool& operator=(const HostPool&) = delete;
-    // fn(0) .. fn(count - 1), each once, in any order; returns when all are
-    // done. fn must not throw.
-    template <typename F> void run(int count, F&& fn) {
-        if (threads_.empty() || count < 2) {
-            for (int i = 0; i < count; ++i) fn(i);
-            return;
-        }
-        auto call = [](void* f, int i) { (*static_cast<std::remove_reference_t<F>*>(f))(i); };
-        {
-            std::lock_guard<std::mutex> l(lock_);
-            call_ = call;
-            arg_ = &fn;
-            count_ = count;
-            next_ = 0;
-            left_ = count;
-        }
-        start_.notify_all();
-        drain();
-        std::unique_lock<std::mutex> l(lock_);
-        done_.wait(l, [this] { return left_ == 0; });
-    }
-
-  private:
-    void drain() {
-        for (;;) {
-            int i;
-            {
-                std::lock_guard<std::mutex> l(lock_);
-                if (next_ >= count_) return;
-                i = next_++;
-            }
-            call_(arg_, i);
-            std::lock_guard<std::mutex> l(lock_);
-            if (--left_ == 0) done_.notify_one();
-        }
-    }
-    void work() {
-        for (;;) {
-            {
-                std::unique_lock<std::mutex> l(lock_);
-                start_.wait(l, [this] { return stop_ || next_ < count_; });
-                if (stop_) return;
-            }
-            drain();
-        }
-    }
-    std::vector<std::thread> threads_;
-    std::mutex lock_;
-    std::condition_variable start_, done_;
-    void (*call_)(void*, int) = nullptr;
-    void* arg_ = nullptr;
-    int count_ = 0, next_ = 0, left_ = 0;
-    bool stop_ = false;
-};
 
 constexpr double kSceneWaves = 4.0;  // multi-scene grids: waves of CTA shares
 template <typename R, typename S, bool ADJ, bool MS = false>
