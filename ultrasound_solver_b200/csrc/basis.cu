@@ -150,7 +150,7 @@ static const int kBasisChunk = 8192;
 // GPU several times over.
 static long long adjoint_chunk(long long n) { return n <= 262144 ? 2048 : kBasisChunk; }
 // Columns per CTA: four when that still leaves four CTAs per SM.
-static bool four_columns(long long nblk, int m) { return nblk * ((m + 3) / 4) >= 4 * 148; }
+static bool four_columns(long long nblk, int m, int sms) { return nblk * ((m + 3) / 4) >= 4LL * sms; }
 
 }  // namespace usv
 
@@ -196,7 +196,10 @@ int usv_basis_adjoint(const void* basis, int64_t n, int m, int prec, const void*
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     double2* part = static_cast<double2*>(workspace);
     const double2* cot = static_cast<const double2*>(cotangent);
-    const bool four = four_columns(nblk, m);
+    int dev = 0, sms = 0;
+    USV_CUDA_TRY(cudaGetDevice(&dev));
+    USV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const bool four = four_columns(nblk, m, sms);
     const dim3 grid(nblk, four ? (m + 3) / 4 : m);
     if (prec == USV_PREC_MIXED) {
         const float2* G = static_cast<const float2*>(basis);
