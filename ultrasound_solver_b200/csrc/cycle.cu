@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
             const int gr = task / segs, sg = task - gr * segs;
             const int q0 = sg * per_seg, q1 = min(units, q0 + per_seg);
             const uint4* vp[kDotVecs];
-            MT acc[2 * kDotVecs];  // (bfloat16: at most 128 nodes per fp32 lane sum, see seg_table)
+            MT acc[2 * kDotVecs];  // (bfloat16: at most 128 nodes per fp32 lane sum, see cycle_segments)
 #pragma unroll
             for (int i = 0; i < kDotVecs; ++i) {
                 const int t = min(gr * kDotVecs + i, nd - 1);  // (a repeated vector's sums are not used)
@@ -540,7 +540,8 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_cycle(OpView<R> op, S* V, GS
             if (threadIdx.x == 0) g.status[b] = ST_DEVICE_TIMEOUT;
             return;
         }
-        // ---- what ||u_j|| decides
+        // ---- what ||u_j|| decides (before any use of hs: the sums over a u_j
+        // that is not finite are meaningless, see widen_scaled)
         double ratio = 1.0, sigma_j = sig[j];
         if (pending) {
             const double n2 = raw_norm, beta = sqrt(n2);

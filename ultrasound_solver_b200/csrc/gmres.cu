@@ -656,8 +656,8 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
         for (int task = warp; task < tasks_t * segs; task += nw) {
             const int t = task / segs, seg = task % segs;
             const int q0 = seg * per_seg, q1 = min(ngroups, q0 + per_seg);
-            // lane sums in the pass arithmetic (fp32 for bfloat16, <= 64 terms
-            // per lane and chunk), FP64 from the warp reduction on
+            // lane sums in the pass arithmetic (fp32 for bfloat16, at most 128
+            // nodes per lane and chunk), FP64 from the warp reduction on
             using MT = typename MathT<C2>::T;
             using M2 = typename MathT<C2>::T2;
             MT lre = 0, lim = 0;

@@ -152,9 +152,9 @@ __device__ __forceinline__ CycleBasis<S> cycle_basis(S* V, const GState& g, int 
 
 // Arithmetic of the basis passes per storage type. bfloat16 values (8-bit
 // mantissa) are combined in fp32: their products, the orthogonalisation
-// update and per-lane partial sums of at most a few dozen terms are far more
-// precise than the stored values; every reduction across lanes, CTAs and
-// chunks stays FP64. complex64 and complex128 bases use FP64 throughout.
+// update and per-lane partial sums (at most 128 nodes, 256 products per part:
+// a 4096-node segment) are far more precise than the stored values; every
+// reduction across lanes, CTAs and chunks stays FP64. complex64 and complex128 bases use FP64 throughout.
 // (Widening to FP64 costs conversion-unit throughput: with bfloat16 the FP64
 // dots saturated that unit in the Arnoldi kernel.)
 template <typename C2> struct MathT {
@@ -183,8 +183,11 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
 // included). Integer instructions: F2F.F64.F32 runs at 16 lanes per clock and
 // SM and bounded the complex64 passes (2 per value and pass). The other factor
 // of a product carries 2^896, or the sum is scaled back. Infinities and NaN
-// would turn finite here: only basis vectors whose norm has been found finite
-// are read this way; w is converted by F2F, once per step.
+// turn finite here, so sums over a basis vector formed this way only count once
+// its norm, from the unscaled values, has been found finite. The per-pass
+// kernels know it before; in the cycle kernel it arrives with the sums of the
+// newest vector, and they are dropped if it is not. w is converted by F2F, once
+// per step.
 __device__ __forceinline__ double widen_scaled(unsigned f) {
     const long long t = (long long)(int)f * (1LL << 29);
     return __hiloint2double(int(t >> 32) & int(0x8fffffff), int(t));
