@@ -343,9 +343,53 @@ __global__ void __launch_bounds__(256, 4) k_apply_kc(OpView<float> op, const flo
 // rows j of plane k. The R right-hand sides (nrhs rounded up to a power of
 // two) are split into G = R / NB groups of NB; a thread applies its node's
 // coefficients to the NB vectors b = g, g + G, ..., and each warp holds 32
-// consecutive nodes (coalesced loads and stores). The rows' coefficients (48
-// bytes per node, contiguous along x) reach shared memory by bulk copies while
-// the threads load their vector values: read by the lanes themselves, 48 bytes
+// consecutive nodes (coalesced loads and stores). Two forms, by size (see
+// bulk_rows_pay):
+//
+// k_apply_kc_direct, for operands that stay in L2: the lanes load their node's
+// coefficients themselves, and the G warps of a row share them through L1.
+template <int R, int NB>
+__global__ void __launch_bounds__(256) k_apply_kc_direct(OpView<float> op, const float2* __restrict__ x,
+                                                         float2* __restrict__ y, long long ld, int nrhs) {
+    constexpr int G = R / NB, kRows = 8 / G;
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    const int g = threadIdx.y % G;
+    const int j = blockIdx.y * kRows + threadIdx.y / G;
+    const int k = blockIdx.z;
+    if (i >= op.nx || j >= op.ny || g >= nrhs) return;
+    const long long sy = op.nx, sz = (long long)op.nx * op.ny;
+    const long long n = i + sy * j + sz * k;
+    const float4* cf = op.cf + 3 * n;
+    const float4 c01 = __ldg(cf), c23 = __ldg(cf + 1), c45 = __ldg(cf + 2);
+    const long long o0 = i > 0 ? -1 : 0, o1 = i < op.nx - 1 ? 1 : 0;
+    const long long o2 = j > 0 ? -sy : 0, o3 = j < op.ny - 1 ? sy : 0;
+    const long long o4 = k > 0 ? -sz : 0, o5 = k < op.nz - 1 ? sz : 0;
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int b = g + G * q;
+        if (b < nrhs) {
+            const float2* xb = x + b * ld + n;
+            float2 v = __ldg(xb);
+            const float2 u0 = __ldg(xb + o0), u1 = __ldg(xb + o1), u2 = __ldg(xb + o2);
+            const float2 u3 = __ldg(xb + o3), u4 = __ldg(xb + o4), u5 = __ldg(xb + o5);
+            auto mac = [&](float cr, float ci, float2 u) {
+                v.x = fmaf(cr, u.x, fmaf(-ci, u.y, v.x));
+                v.y = fmaf(cr, u.y, fmaf(ci, u.x, v.y));
+            };
+            mac(c01.x, c01.y, u0);
+            mac(c01.z, c01.w, u1);
+            mac(c23.x, c23.y, u2);
+            mac(c23.z, c23.w, u3);
+            mac(c45.x, c45.y, u4);
+            mac(c45.z, c45.w, u5);
+            y[b * ld + n] = v;
+        }
+    }
+}
+
+// k_apply_kc_rhs, for operands from DRAM: the rows' coefficients (48 bytes per
+// node, contiguous along x) reach shared memory by bulk copies while the
+// threads load their vector values: read by the lanes themselves, 48 bytes
 // apart, they took most of the L1 path that bounds this kernel, once per group.
 // 128^3, per launch: 33.2 -> 29.0 us (2 right-hand sides), 49.6 -> 45.3 (4,
 // 5.2 TB/s), 94.8 -> 82.0 (8). Marching through z with the column's values in
@@ -411,6 +455,19 @@ __global__ void __launch_bounds__(256) k_apply_kc_rhs(OpView<float> op, const fl
         }
     }
 }
+
+// Coefficients by bulk copies once the operands (48 bytes of coefficients and
+// 16 per right-hand side and node) take more than 0.7 of the L2 (93 of 133e6
+// bytes). Below, a launch finds them in L2 when it is repeated, and the
+// wait for the copies costs more than the lanes' loads. Direct / bulk, us:
+//   1 right-hand side   4.8 / 6.3 at 17 MB, 8.5 / 10.4 at 64, 12.5 / 14.4 at 90, 18.7 / 18.7 at 111
+//   2                   6.4 / 8.4 at 31 MB, 10.5 / 12.4 at 71, 16.7 / 16.9 at 90, 24.8 / 22.7 at 112
+//   3                   6.4 / 8.4 at 25 MB, 10.5 / 12.4 at 49, 16.8 / 16.6 at 85, 24.7 / 22.7 at 96
+//   4                   8.3 / 9.5 at 36 MB, 18.9 / 18.7 at 81, 22.8 / 20.7 at 99, 33.0 / 30.6 at 126
+//   8                   16.6 / 15.6 at 69 MB, 28.0 / 24.9 at 90, 43.2 / 37.2 at 128
+// (Operands that are not in L2 yet: the bulk form is up to 15% faster at all
+// these sizes.)
+static bool bulk_rows_pay(long long n, int nrhs, int l2) { return 10 * n * (48 + 16LL * nrhs) > 7LL * l2; }
 
 // y = K x through the z-marching tile kernel (usv_internal.cuh: zmarch_rows):
 // usv_operator_apply K / K^H in complex128 (74 us at 128^3 against 97 us for a
@@ -730,10 +787,20 @@ int usv_operator_apply_kernel(const usv_scene* scene, const void* op_buf, int va
                     const float2* xf = (const float2*)x;
                     float2* yf = (float2*)y;
                     const int r = nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : nrhs <= 4 ? 4 : 8;
-                    const int rows = r == 8 ? 4 : 8;  // rows of a CTA: 8 / groups
+                    int dev = 0, l2 = 0;
+                    USV_CUDA_TRY(cudaGetDevice(&dev));
+                    USV_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+                    const bool bulk = bulk_rows_pay(v.n, nrhs, l2);
+                    // rows of a CTA: 8 / groups
+                    const int rows = bulk ? (r == 8 ? 4 : 8) : (r == 8 ? 2 : r == 4 ? 4 : 8);
                     const dim3 g3((s.nx + 31) / 32, (s.ny + rows - 1) / rows, s.nz);
                     const dim3 b3(32, 8);
-                    if (r == 1) k_apply_kc_rhs<1, 1><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
+                    if (!bulk) {
+                        if (r == 1) k_apply_kc_direct<1, 1><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
+                        else if (r == 2) k_apply_kc_direct<2, 2><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
+                        else if (r == 4) k_apply_kc_direct<4, 2><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
+                        else k_apply_kc_direct<8, 2><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
+                    } else if (r == 1) k_apply_kc_rhs<1, 1><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
                     else if (r == 2) k_apply_kc_rhs<2, 2><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
                     else if (r == 4) k_apply_kc_rhs<4, 4><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
                     else k_apply_kc_rhs<8, 4><<<g3, b3, 0, strm>>>(v, xf, yf, ld, nrhs);
