@@ -244,3 +244,25 @@ def test_loss_many_targets():
         loss = -1.5 * u[t].abs().mean() + 0.05 * (u.abs() ** 2).mean()
         assert abs(float(value[0] - loss)) < 1e-12
         assert float((cot - want).abs().max()) < 1e-14
+
+
+@pytest.mark.parametrize("n,m", [(1000, 1), (65536, 7), (65536, 8), (65537, 8), (65537, 16), (300001, 31),
+                                 (300001, 33), (800001, 40)])
+@pytest.mark.parametrize("precision", ["complex64", "complex128"])
+def test_basis_field_forms(n, m, precision):
+    """Plain and eight-column form by size, remainders among them: the same
+    column order, so at most the rounding of m fused products (1e-15 m)."""
+    from ultrasound_solver_b200 import _native as N
+    dtype = getattr(torch, precision)
+    prec = N.PREC_MIXED if precision == "complex64" else N.PREC_FP64
+    gen = torch.Generator(device="cuda").manual_seed(n + m)
+    G = torch.randn(m, n, dtype=dtype, device="cuda", generator=gen)
+    ph = torch.rand(m, dtype=torch.float64, device="cuda", generator=gen)
+    out = torch.empty(n, dtype=torch.complex128, device="cuda")
+    N.check(N.load().usv_basis_field(N.ptr(G), n, m, prec, N.ptr(ph), N.ptr(out), N.stream_handle(torch, G.device)))
+    want = torch.zeros(n, dtype=torch.complex128, device="cuda")
+    scale = torch.zeros(n, dtype=torch.float64, device="cuda")
+    for g, p in zip(G, ph):
+        want += g.to(torch.complex128) * torch.exp(1j * p)
+        scale += g.abs()
+    assert float(((out - want).abs() / scale).max()) < 1e-15 * (m + 4)

@@ -9,9 +9,9 @@
 
 namespace usv {
 
-constexpr int kFieldCols = 8;
-
-template <typename C2>
+// COLS columns in flight per thread (1: left to the compiler). The sum runs in
+// column order in both forms.
+template <typename C2, int COLS>
 __global__ void __launch_bounds__(256) k_field(const C2* G, long long N, int M,
                                                const double* phases, double2* out) {
     extern __shared__ double2 w[];
@@ -25,15 +25,19 @@ __global__ void __launch_bounds__(256) k_field(const C2* G, long long N, int M,
          n += (long long)gridDim.x * blockDim.x) {
         double2 acc = make_double2(0.0, 0.0);
         const C2* col = G + n;
-        int m = 0;
-        for (; m + kFieldCols <= M; m += kFieldCols) {  // kFieldCols columns in flight
-            C2 v[kFieldCols];
+        if constexpr (COLS == 1) {
+            for (int m = 0; m < M; ++m) acc = cadd(acc, cmul(to_d(col[(long long)m * N]), w[m]));
+        } else {
+            int m = 0;
+            for (; m + COLS <= M; m += COLS) {
+                C2 v[COLS];
 #pragma unroll
-            for (int q = 0; q < kFieldCols; ++q) v[q] = col[(long long)(m + q) * N];
+                for (int q = 0; q < COLS; ++q) v[q] = col[(long long)(m + q) * N];
 #pragma unroll
-            for (int q = 0; q < kFieldCols; ++q) acc = cadd(acc, cmul(to_d(v[q]), w[m + q]));
+                for (int q = 0; q < COLS; ++q) acc = cadd(acc, cmul(to_d(v[q]), w[m + q]));
+            }
+            for (; m < M; ++m) acc = cadd(acc, cmul(to_d(col[(long long)m * N]), w[m]));
         }
-        for (; m < M; ++m) acc = cadd(acc, cmul(to_d(col[(long long)m * N]), w[m]));
         out[n] = acc;
     }
 }
@@ -144,6 +148,23 @@ static unsigned grid1(long long n) {
     return unsigned(b < 1 ? 1 : b);
 }
 
+// Eight columns in flight where the loads' latency is what a thread waits for:
+// small grids, and longer sums. Few columns, and complex64 grids whose columns
+// come from DRAM, are faster with the plain loop (its registers leave room for
+// more threads). Plain / eight, us:
+//   complex64   n =  63000: m = 8 4.2 / 4.2, 13 6.2 / 4.9, 64 12.5 / 10.3, 256 97 / 73
+//               n = 262144: m = 3 5.0 / 6.2, 16 8.4 / 8.3, 64 53 / 41, 256 193 / 147
+//               n = 512000: m = 7 8.3 / 10.3, 16 12.4 / 14.3, 64 78.6 / 77.8, 256 291 / 283
+//               n = 723456: m = 36 59.5 / 57.8, 256 389 / 361
+//               n = 884736: m = 7 10.4 / 14.4, 36 63.6 / 69.5, 256 405 / 436
+//   complex128  n =  63000: m = 16 6.2 / 5.0, 256 78 / 60
+//               n = 262144: m = 2 4.5 / 6.3, 16 10.0 / 8.3, 256 181 / 158
+//               n = 884736: m = 7 20.9 / 26.7, 16 41.6 / 41.1, 64 137.5 / 135.2
+static bool eight_columns(long long n, int m, size_t bytes) {
+    if (n <= 65536) return m >= 8;
+    return bytes == 16 ? m >= 16 : m >= 32 && n <= 800000;
+}
+
 static const int kBasisChunk = 8192;
 // Nodes per CTA of usv_basis_adjoint. A CTA of 8192 nodes is 32 dependent
 // passes of its 256 threads, too long a chain when the basis does not fill the
@@ -162,15 +183,20 @@ int usv_basis_field(const void* basis, int64_t n, int m, int prec, const double*
                     void* field, void* stream) {
     if (!basis || n < 1 || m < 1 || m > 3072 || !phases || !field) return USV_ERR_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const size_t smem = sizeof(double2) * m;
-    if (prec == USV_PREC_MIXED)
-        k_field<float2><<<grid1(n), 256, smem, s>>>(static_cast<const float2*>(basis), n, m,
-                                                    phases, static_cast<double2*>(field));
-    else if (prec == USV_PREC_FP64)
-        k_field<double2><<<grid1(n), 256, smem, s>>>(static_cast<const double2*>(basis), n, m,
-                                                     phases, static_cast<double2*>(field));
-    else
-        return USV_ERR_ARG;
+    if (prec != USV_PREC_MIXED && prec != USV_PREC_FP64) return USV_ERR_ARG;
+    const size_t smem = sizeof(double2) * m, bytes = prec == USV_PREC_MIXED ? sizeof(float2) : sizeof(double2);
+    const bool eight = eight_columns(n, m, bytes);
+    double2* out = static_cast<double2*>(field);
+    const unsigned grid = grid1(n);
+    if (prec == USV_PREC_MIXED) {
+        const float2* G = static_cast<const float2*>(basis);
+        if (eight) k_field<float2, 8><<<grid, 256, smem, s>>>(G, n, m, phases, out);
+        else k_field<float2, 1><<<grid, 256, smem, s>>>(G, n, m, phases, out);
+    } else {
+        const double2* G = static_cast<const double2*>(basis);
+        if (eight) k_field<double2, 8><<<grid, 256, smem, s>>>(G, n, m, phases, out);
+        else k_field<double2, 1><<<grid, 256, smem, s>>>(G, n, m, phases, out);
+    }
     USV_CUDA_TRY(cudaGetLastError());
     return USV_OK;
 }
