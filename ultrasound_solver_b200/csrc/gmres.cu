@@ -599,6 +599,7 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
         segsum[task] = make_double2(0.0, 0.0);
     const int nphase = int((N + DC - 1) / DC);
     const int keep_from = nphase - l2_chunks<C2, DC>(g, j);
+    const unsigned long long coef_pol = g.coef_keep ? l2_evict_normal() : l2_evict_first();
     for (int ch = blockIdx.x, par = 0; ch < nphase; ch += ncta, par ^= NBUF - 1) {
         const long long n0 = (long long)ch * DC;
         const int len = int(min((long long)DC, N - n0));
@@ -624,8 +625,8 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
                     C2 y = from_d<C2>(make_double2(0.0, 0.0));
                     if (e < len) {
                         const long long n = n0 + e;
-                        y = narrow<C2>(cscale(rows16 ? k_row_cb_clamped(op, uj, n)
-                                                     : k_row_cf_clamped(op, uj, n), sj));
+                        y = narrow<C2>(cscale(rows16 ? k_row_cb_clamped(op, uj, n, coef_pol)
+                                                     : k_row_cf_clamped(op, uj, n, coef_pol), sj));
                         w[n] = y;
                     }
                     ys[e] = as_ys<YS>(y);
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(NT, 2) k_dots(OpView<R> op, S* V, GState g, in
                     C2 y = from_d<C2>(make_double2(0.0, 0.0));
                     if (e < len) {
                         const long long n = n0 + e;
-                        y = narrow<C2>(cscale(k_row<R, ADJ, S>(op, uj, n, p), sj));
+                        y = narrow<C2>(cscale(k_row<R, ADJ, S>(op, uj, n, p, coef_pol), sj));
                         w[n] = y;
                     }
                     ys[Place::at(e)] = as_ys<YS>(y);
@@ -2319,6 +2320,13 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
     int l2 = 0;
     USV_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
     g.l2_keep = (long long)l2 * 2 / 5;
+    // A basis that leaves room in L2 for the row coefficients keeps them, up to
+    // two thirds of the L2 together. No hints / coefficients first out / kept
+    // (five cycles of GMRES(30), bfloat16, ms): 56^3 4.55 / 4.76 / 4.55,
+    // 80^3 5.34 / 5.71 / 5.43, 88^3 6.45 / 6.61 / 6.65.
+    const double coef_bytes = double(g.n) * (MS ? B : 1) * (sizeof(R) == 8 ? 32 : sizeof(C2) == 4 ? 24 : 48);
+    const double pass_bytes = double(B) * (g.m + 1) * double(g.nv) * sizeof(C2) + coef_bytes;
+    g.coef_keep = pass_bytes <= double(l2) * 2 / 3;
     auto grid_for = [&](const void* fn, int threads, size_t smem, dim3& grid,
                         int fixed_per_sm = 0) -> int {
         int per_sm = fixed_per_sm;

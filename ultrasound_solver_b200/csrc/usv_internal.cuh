@@ -426,9 +426,8 @@ __device__ __forceinline__ void k_coefs_from(const OpView<float>& op, Node p, fl
 // coefficient, so their loads are redirected to u_n, which exists and is finite.
 template <typename S>
 __device__ __forceinline__ float2 k_row_cf(const OpView<float>& op, const S* __restrict__ u,
-                                           long long n, Node p) {
+                                           long long n, Node p, unsigned long long pol) {
     const float4* c = op.cf + 3 * n;
-    const unsigned long long pol = l2_evict_first();
     const float4 c01 = ldg16(c, pol), c23 = ldg16(c + 1, pol), c45 = ldg16(c + 2, pol);
     const long long sy = op.nx, sz = (long long)op.nx * op.ny;
     const float2 u0 = widen<float2>(u[p.i > 0 ? n - 1 : n]);
@@ -456,10 +455,9 @@ __device__ __forceinline__ float2 k_row_cf(const OpView<float>& op, const S* __r
 // the same vector. Equal to k_row_cf wherever u is finite (a zero coefficient
 // times a finite value adds zero).
 template <typename S>
-__device__ __forceinline__ float2 k_row_cf_clamped(const OpView<float>& op,
-                                                   const S* __restrict__ u, long long n) {
+__device__ __forceinline__ float2 k_row_cf_clamped(const OpView<float>& op, const S* __restrict__ u, long long n,
+                                                   unsigned long long pol) {
     const float4* c = op.cf + 3 * n;
-    const unsigned long long pol = l2_evict_first();
     const float4 c01 = ldg16(c, pol), c23 = ldg16(c + 1, pol), c45 = ldg16(c + 2, pol);
     const long long sy = op.nx, sz = (long long)op.nx * op.ny, last = op.n - 1;
     const float2 u0 = widen<float2>(u[n > 0 ? n - 1 : 0]);
@@ -485,10 +483,9 @@ __device__ __forceinline__ float2 k_row_cf_clamped(const OpView<float>& op,
 // The bfloat16 row from the packed bfloat16 coefficients: every product
 // c_d u_d is bf16 x bf16, exact in fp32 (fma.rn.f32.bf16), summed in fp32;
 // clamped neighbour indices as above.
-__device__ __forceinline__ float2 k_row_cb_clamped(const OpView<float>& op,
-                                                   const bf2* __restrict__ u, long long n) {
+__device__ __forceinline__ float2 k_row_cb_clamped(const OpView<float>& op, const bf2* __restrict__ u, long long n,
+                                                   unsigned long long pol) {
     const uint2* c = op.cb + 3 * n;
-    const unsigned long long pol = l2_evict_first();
     const uint2 c01 = ldg8(c, pol), c23 = ldg8(c + 1, pol), c45 = ldg8(c + 2, pol);
     const long long sy = op.nx, sz = (long long)op.nx * op.ny, last = op.n - 1;
     const unsigned* w = reinterpret_cast<const unsigned*>(u);
@@ -509,11 +506,11 @@ __device__ __forceinline__ float2 k_row_cb_clamped(const OpView<float>& op,
 
 template <typename R, bool ADJ, typename S = typename Tr<R>::c2>
 __device__ __forceinline__ typename Tr<R>::c2 k_row(const OpView<R>& op, const S* __restrict__ u,
-                                                    long long n, Node p) {
+                                                    long long n, Node p, unsigned long long pol) {
     using C2 = typename Tr<R>::c2;
     using C4 = typename Tr<R>::c4;
     if constexpr (sizeof(R) == 4) {
-        return k_row_cf(op, u, n, p);
+        return k_row_cf(op, u, n, p, pol);
     } else {
         const C2 un = widen<C2>(u[n]);
         if (!ADJ && node_fixed(op.soft, p.i, p.j, p.k, op.nx, op.ny, op.nz)) return un;
