@@ -884,8 +884,11 @@ __global__ void __launch_bounds__(kThreads) k_orth(S* V, long long N, GState g, 
     __syncthreads();  // hs, hm visible
     double acc = 0.0;
     // last chunk first: the dots pass ended there, and what it read last is
-    // still in L2 (the next dots pass starts where this one ends)
-    for (int ch = nchunk - 1 - int(blockIdx.x); ch >= 0; ch -= ncta) {
+    // still in L2 (the next dots pass starts where this one ends). First chunk
+    // first for complex128 bases of the size of the L2, see run_gmres.
+    const bool forward = sizeof(C2) == 16 && g.orth_forward;
+    for (int q = blockIdx.x; q < nchunk; q += ncta) {
+        const int ch = forward ? q : nchunk - 1 - q;
         const long long n0 = (long long)ch * kChunk;
         const int len = int(min((long long)kChunk, N - n0));
         C2* w = cb.V + (long long)(j + 1) * g.nv + n0;
@@ -2327,6 +2330,12 @@ static int run_gmres(const usv_scene& s, const void* op_buf, const usv_gmres_par
     const double coef_bytes = double(g.n) * (MS ? B : 1) * (sizeof(R) == 8 ? 32 : sizeof(C2) == 4 ? 24 : 48);
     const double pass_bytes = double(B) * (g.m + 1) * double(g.nv) * sizeof(C2) + coef_bytes;
     g.coef_keep = pass_bytes <= double(l2) * 2 / 3;
+    // The complex128 orthogonalisation (no hints on its loads) runs against the
+    // dots' order only where the basis is far larger than L2. Both passes in
+    // order / this one backwards (five cycles of GMRES(30), ms): 95 MB 6.26 /
+    // 6.78, 162 MB 9.17 / 10.1, 260 MB 10.7 / 11.0, 285 MB 11.6 / 11.8, 321 MB
+    // 16.1 / 15.4, 354 MB 16.5 / 16.0, 488 MB 19.8 / 19.6.
+    g.orth_forward = pass_bytes <= double(l2) * 9 / 4;
     auto grid_for = [&](const void* fn, int threads, size_t smem, dim3& grid,
                         int fixed_per_sm = 0) -> int {
         int per_sm = fixed_per_sm;

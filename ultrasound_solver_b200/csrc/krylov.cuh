@@ -80,6 +80,7 @@ struct GState {
     unsigned long long* cyc_epoch;  // step number before the next launch
     long long l2_keep; // bytes of a basis pass that the next pass is to find in L2
     int coef_keep;     // 1: the row coefficients as well
+    int orth_forward;  // 1: k_orth walks the node chunks in the order of the dots
     const struct SceneSlot* slots;  // [B] multi-scene solves: the scene of each RHS
 };
 
