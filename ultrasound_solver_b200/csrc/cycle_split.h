@@ -56,23 +56,22 @@ constexpr int cycle_instances(int bytes, bool scenes) { return bytes == 16 ? 2 :
 constexpr int cycle_units(int bytes, int i) { return (bytes == 16 ? 2 : 1) << i; }  // 16-byte loads per thread
 constexpr int cycle_capacity(int bytes, int i) { return kCycThreads * (16 / bytes) * cycle_units(bytes, i); }
 
-// Most nodes per CTA for which the cycle kernel is taken. Alone it is the
-// faster one up to 12288, 7104 and 2496 nodes, per Arnoldi step of GMRES(30),
-// cycle kernel / one launch per pass (us; nodes over all right-hand sides):
-//   bfloat16   23.9 / 40.0 at 593 k, 34.2 / 49.6 at 1.00 M, 61.9 / 63.8 at 1.40 M, 71.8 / 73.1 at 1.73 M,
+// Most nodes per CTA for which the cycle kernel is taken. Alone, per Arnoldi
+// step of GMRES(30), cycle kernel / one launch per pass (us; nodes over all
+// right-hand sides):
+//   bfloat16   22.7 / 36.0 at 593 k, 34.0 / 46.5 at 1.00 M, 61.9 / 63.8 at 1.40 M, 71.8 / 73.1 at 1.73 M,
 //              72.7 / 72.5 at 1.82 M, 78.6 / 76.4 at 1.91 M, 84.3 / 78.7 at 2.10 M
-//   complex64  33.2 / 46.4 at 524 k, 60.4 / 65.1 at 729 k, 77.4 / 78.3 at 1.00 M, 72.8 / 72.8 at 1.05 M (4 x 64^3),
+//   complex64  32.6 / 46.0 at 512 k, 60.4 / 65.1 at 729 k, 77.4 / 78.3 at 1.00 M, 72.8 / 72.8 at 1.05 M (4 x 64^3),
 //              84.3 / 80.0 at 1.12 M, 81.9 / 76.6 at 1.19 M
-//   complex128 30.2 / 50.8 at 262 k, 59.2 / 64.8 at 314 k, 61.7 / 67.0 at 365 k (4 x 45^3),
-//              68.2 / 68.2 at 373 k, 75.0 / 71.2 at 405 k
-// where the basis is far larger than L2 and both read it from DRAM. But its
-// launches hold the shared memory of their SMs, so those of solves on other
-// streams wait, while per-pass kernels overlap. Solves at once, each on its own
-// stream, ms (2 / 8 solves):
+//   complex128 29.2 / 47.1 at 262 k, 32.3 / 49.3 at 287 k, 59.2 / 55.9 at 314 k, 61.7 / 58.6 at 365 k (4 x 45^3)
+// The basis is then far larger than L2 and both read it from DRAM. But the
+// kernel's launches hold the shared memory of their SMs, so those of solves on
+// other streams wait, while per-pass kernels overlap. Solves at once, each on
+// its own stream, ms (2 / 8 solves):
 //   bfloat16   104^3 22.4 / 88 against 23.1 / 93, 112^3 34.6 / 141 against 28.7 / 123 (GMRES(30)),
 //              104^3 40.2 / 161 against 40.4 / 163, 112^3 62.6 / 253 against 49.6 / 198 (GCRO-DR(36,8))
 //   complex64  84^3 22.8 / 90 against 23.0 / 97, 88^3 32.6 / 129 against 27.3 / 119
-//   complex128 66^3 18.8 / 77 against 23.2 / 95, 68^3 34.0 / 137 against 27.4 / 115
+//   complex128 66^3 19.5 / 77 against 23.8 / 86, 68^3 34.0 / 137 against 27.0 / 108
 // So one scene goes as far as it wins both ways: 8192, 4096 and 2048 nodes. A
 // batch of scenes is itself the overlap; two batches at once (100 iterations)
 // took 25.4 ms against 25.1 (bfloat16, 1.59 M nodes), 17.4 against 20.4
